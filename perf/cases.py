@@ -191,7 +191,11 @@ def run(state):
         return {"x": x, "y": y, "iterations": iterations}
     if kind == "jrp":
         state.solver.run()
-        return _jrp_result(state.solver.result(want_solution=case["solution"]))
+        out = _jrp_result(state.solver.result(want_solution=case["solution"]))
+        if case["solution"] and case["precision"] == "mixed":
+            # FP32 iterates come back widened; they are kept as they are
+            out |= {k: out[k].astype(np.float32) for k in "xyz"}
+        return out
     if kind == "jrp_oneshot":
         return _jrp_result(state.library.solve(state.inst, state.params, precision=case["precision"],
                                                want_solution=True))
