@@ -976,6 +976,110 @@ __device__ __forceinline__ void tiny_lower(const Dev<Real>& d, const Real* ys, c
     }
 }
 
+// The plain steps (no check sums) of a solve whose arrays all sit in shared
+// memory: node_kernel_tile's and edge_kernel_tile's arithmetic, term for term,
+// with nothing tied to the graph's tiles.  These steps are a chain of dependent
+// latencies, so the chain is what the split shortens: two threads a node add
+// its two runs side by side, four values of a run at a time; a step's Halpern
+// weights (four FP64 divisions) are made for kStepTable steps at once by as
+// many threads; the edges are dealt to all threads, and every address is a
+// shared-memory one.  A plain step at n = 200, m = 1,000 takes 2,500 cycles
+// (FP32; 3,350 in FP64) and the solve 0.206 / 0.242 ms, against 0.31 / 0.34 ms
+// with the check steps' code for every step; what is left is the latency of a
+// step's two phases and, half of it, the checks.
+constexpr int kStepTable = 64;
+template <class Real>
+struct StepWeights {   // x's combination at this step, and the dual's at the next
+    Real lw, rw, lwn, rwn;
+};
+template <class Real>
+__device__ __forceinline__ StepWeights<Real> step_weights(long long since, int step) {
+    const double k = double(since + step + 1), kn = double(since + step + 2);
+    return {Real(k / (k + 1.0)), Real(1.0 / (k + 1.0)), Real(kn / (kn + 1.0)), Real(1.0 / (kn + 1.0))};
+}
+
+// Unconditional shared-memory load: a plain load under a select may become a
+// branch of its own that waits for it.
+__device__ __forceinline__ unsigned shared_address(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
+template <class Real>
+__device__ __forceinline__ Real load_shared(unsigned at) {
+    Real v;
+    if constexpr (sizeof(Real) == 4) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at));
+    else asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(at));
+    return v;
+}
+
+// v[k .. e) added in order from zero; v in shared memory.  (A value past the
+// end adds zero, which changes no sum's bits.)
+template <class Real>
+__device__ __forceinline__ Real shared_run(const Real* v, int k, int e) {
+    constexpr int U = 4;
+    const unsigned at = shared_address(v);
+    Real s = Real(0);
+    for (; k < e; k += U) {
+        Real t[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) t[u] = load_shared<Real>(at + unsigned(min(k + u, e - 1)) * unsigned(sizeof(Real)));
+#pragma unroll
+        for (int u = 0; u < U; ++u) s += k + u < e ? t[u] : Real(0);
+    }
+    return s;
+}
+
+template <class Real>
+struct TinyView {   // the instance and iterates in this CTA's shared memory
+    int n, m;
+    Real *x1, *x2, *x0, *r, *pred, *pred1, *u0;
+    const Real *diag, *deg, *w;
+    const int *row_ptr, *col_ptr, *colpos;
+    const int2* ends;
+    int* status;
+};
+
+template <class Real>
+__device__ __forceinline__ void tiny_node_plain(const TinyView<Real>& t, Real lw, Real rw, Real ps) {
+    const int half = threadIdx.x & 1;
+    const int* const ptr = half ? t.col_ptr : t.row_ptr;
+    const Real* const v = half ? t.pred1 : t.pred;
+    for (int base = 0; base < t.n; base += int(blockDim.x) / 2) {
+        const int i = base + int(threadIdx.x >> 1);
+        Real s = Real(0);
+        if (i < t.n) {
+            const int k = ptr[i], e = ptr[i + 1];
+            if (index_ok(0 <= k && k <= e && e <= t.m, t.status)) s = shared_run<Real>(v, k, e);
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if (i < t.n && !half) {
+            const Real x2o = t.x2[i], x1v = rfma(lw, rfma(Real(2), x2o, -t.x1[i]), rmul(rw, t.x0[i]));
+            const Real x2v = clampv(rfma(-ps, (t.diag[i] - s) / t.deg[i], x1v), Real(0), Real(1));
+            t.x1[i] = x1v;
+            t.x2[i] = x2v;
+            t.r[i] = rfma(Real(2), x2v, -x1v);
+        }
+    }
+}
+
+template <class Real>
+__device__ __forceinline__ void tiny_edge_plain(const TinyView<Real>& t, Real lwn, Real rwn, Real hs) {
+#pragma unroll 2
+    for (int e = threadIdx.x; e < t.m; e += blockDim.x) {
+        const int2 ij = t.ends[e];
+        const Real sw = t.w[e], u1 = t.pred[e], u0 = t.u0[e];
+        const int at1 = t.colpos[e];
+        if (!index_ok(unsigned(ij.x) < unsigned(t.n) && unsigned(ij.y) < unsigned(t.n) && unsigned(at1) < unsigned(t.m),
+                      t.status))
+            continue;
+        const Real ri = t.r[ij.x], rj = t.r[ij.y];
+        const bool cov = sw > Real(0);
+        const Real w = cov ? sw : -sw;
+        const Real u2 = cov ? clampv(rfma(hs, (Real(1) - ri) - rj, u1), -w, Real(0))
+                            : clampv(rfma(hs, rj - ri, u1), Real(0), w);
+        const Real nx = rfma(lwn, rfma(Real(2), u2, -u1), rmul(rwn, u0));
+        t.pred[e] = nx;
+        t.pred1[at1] = cov ? nx : w - nx;
+    }
+}
+
 // check_body, out of line: its row reductions hold many values at once, and
 // inlined they would hold registers through the whole step loop.
 __device__ __noinline__ void tiny_check(Control* c, const Params& prm, const double* scale, const double* pnode,
@@ -993,6 +1097,7 @@ tiny_solve_kernel(const __grid_constant__ Dev<Real> g, const __grid_constant__ P
     __shared__ Dev<Real> d;
     __shared__ double scratch[kTinyParts * kEdgeSums * 32];
     __shared__ double qout[kTinyParts * kEdgeSums];
+    __shared__ StepWeights<Real> weights[kStepTable];
     const TinyLayout L = tiny_layout(g.n, g.m, nb_node, nb_edge, int(sizeof(Real)));
     auto at = [&](size_t off) { return static_cast<void*>(smem_raw + off); };
     if (threadIdx.x == 0) {
@@ -1055,22 +1160,47 @@ tiny_solve_kernel(const __grid_constant__ Dev<Real> g, const __grid_constant__ P
         tiny_check(d.ctl, prm, d.scale, d.pnode, nb_node, d.pedge, nb_edge, d.plower, 0);
         __syncthreads();
     }
+    TinyView<Real> view;
+    view.n = g.n;
+    view.m = g.m;
+    view.x1 = static_cast<Real*>(at(L.x1));
+    view.x2 = static_cast<Real*>(at(L.x2));
+    view.x0 = static_cast<Real*>(at(L.x0));
+    view.r = static_cast<Real*>(at(L.r));
+    view.pred = static_cast<Real*>(at(L.pred));
+    view.pred1 = static_cast<Real*>(at(L.pred1));
+    view.u0 = static_cast<Real*>(at(L.u0));
+    view.diag = static_cast<const Real*>(at(L.diag));
+    view.deg = static_cast<const Real*>(at(L.deg));
+    view.w = static_cast<const Real*>(at(L.w));
+    view.row_ptr = static_cast<const int*>(at(L.row_ptr));
+    view.col_ptr = static_cast<const int*>(at(L.col_ptr));
+    view.colpos = static_cast<const int*>(at(L.colpos));
+    view.ends = static_cast<const int2*>(at(L.ends));
+    view.status = &d.ctl->status;
     const int op = int(prm.op_steps);
     for (int b = 0; b < max_blocks && !d.ctl->terminated; ++b) {
         // one check block: enqueue_steps' kernels, in their order
-        for (int s = 0; s < op; ++s) {
-            if (s + 1 < op)
-                tiny_node<Real, true, false>(d, d.pred, d.pred1, s, 0, 0, nb_node, scratch, qout);
-            else
-                tiny_node<Real, true, true>(d, d.pred, d.pred1, s, 0, 0, nb_node, scratch, qout);
-            __syncthreads();
-            if (m) {
-                if (s + 1 < op)
-                    tiny_edge<Real, true, false>(d, nullptr, s, 0, 0, nb_edge, scratch, qout);
-                else
-                    tiny_edge<Real, true, true>(d, nullptr, s, 0, 0, nb_edge, scratch, qout);
+        const double omega = d.ctl->omega;
+        const long long since = d.ctl->restart_iter;
+        const Real ps = Real(kEta / omega), hs = Real(0.5 * kEta * omega);
+        for (int s = 0; s + 1 < op; ++s) {
+            if (s % kStepTable == 0) {
+                __syncthreads();
+                if (threadIdx.x < kStepTable) weights[threadIdx.x] = step_weights<Real>(since, s + int(threadIdx.x));
                 __syncthreads();
             }
+            const StepWeights<Real> sw = weights[s % kStepTable];
+            tiny_node_plain<Real>(view, sw.lw, sw.rw, ps);
+            __syncthreads();
+            tiny_edge_plain<Real>(view, sw.lwn, sw.rwn, hs);
+            __syncthreads();
+        }
+        tiny_node<Real, true, true>(d, d.pred, d.pred1, op - 1, 0, 0, nb_node, scratch, qout);
+        __syncthreads();
+        if (m) {
+            tiny_edge<Real, true, true>(d, nullptr, op - 1, 0, 0, nb_edge, scratch, qout);
+            __syncthreads();
         }
         tiny_lower<Real>(d, d.u2s, d.u2s1, nb_node, scratch, qout);
         __syncthreads();
@@ -1477,16 +1607,16 @@ struct Solver final : SolverBase {
         return set_mega(mode);
     }
 
-    // mode -1: automatic (the single-CTA form for at most kTinyAutoTiles edge
-    // tiles, else the graph: measured per solve, the single-CTA form is 2x
-    // faster than the graph at n = 200-400 and 1.5x at n = 700, m = 2,000,
-    // but 4 % slower at n = 1,500, m = 4,500; the grid form was slower than the
-    // graph from n = 400 up); 0: the graph; 1: the single-CTA form when it
+    // mode -1: automatic (the single-CTA form wherever the instance fits one
+    // CTA's shared memory, else the graph: per solve 0.21 against 0.60 ms at
+    // n = 200, m = 1,000, 0.36 against 0.64 at n = 700, m = 2,800, 1.63 against
+    // 2.01 at n = 1,500, m = 4,500, FP32, and 0.375 against 0.395 at n = 2,500,
+    // m = 3,000, about the largest that fits; the grid form was slower than
+    // the graph from n = 400 up); 0: the graph; 1: the single-CTA form when it
     // fits, else the grid form; 2: the grid form.
-    static constexpr int kTinyAutoTiles = 2;
     cudaError_t set_mega(int mode) {
         mega_mode = mode < 0 ? -1 : (mode > 2 ? 2 : mode);
-        tiny = tiny_fits && (mega_mode == 1 || (mega_mode == -1 && nb_edge <= kTinyAutoTiles));
+        tiny = tiny_fits && (mega_mode == 1 || mega_mode == -1);
         mega = !tiny && mega_mode >= 1 && mega_grid > 0;
         if (mega && !bar.ptr) {
             RB_CUDA_TRY(bar.alloc(1, stream));

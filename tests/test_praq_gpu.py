@@ -482,6 +482,30 @@ def test_persistent_kernel_equals_graph(native, use_float32, shape, form):
     assert ml < gl
 
 
+@pytest.mark.parametrize("use_float32", [0, 1])
+@pytest.mark.parametrize("n,m,op_steps", [(2, 1, 2), (17, 60, 16), (255, 300, 65), (257, 513, 64), (513, 1025, 130),
+                                          (900, 1500, 16)])
+def test_single_cta_plain_steps_equal_graph(native, use_float32, n, m, op_steps):
+    """The single-CTA form's plain steps (two threads a node, four values of a
+    run at a time, a table of 64 steps' weights) against the graph, bit for
+    bit, around the edges of each: one pass of 256 nodes and more, runs that
+    are no multiple of four, blocks of fewer and of more steps than the table."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import DeviceSolver, Library
+    inst = qubo_uniform_edges(n, n, m)
+    p = Library().parameters(tolerance=1e-4 if use_float32 else 1e-8, use_float32=use_float32, max_iter=1000,
+                             op_steps=op_steps)
+    out = {}
+    for mode in (0, 1):
+        with DeviceSolver(inst, p) as dev:
+            assert dev.set_megakernel(mode) == (0 if mode == 0 else 2)
+            assert dev.run() in (0, 1)                 # converged, or the iteration limit
+            out[mode] = dev.result(want_x=True, want_dual=True)
+    (a, ya), (b, yb) = out[0], out[1]
+    assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
+    assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
+
+
 def test_persistent_kernel_choice_and_edgeless(native):
     from reformulation_b200.instances import qubo_uniform_edges
     from reformulation_b200.praq import DeviceSolver, Library
