@@ -148,8 +148,8 @@ REFORM_API int reform_praq_run_profiled(reform_praq_solver* solver, double* ms, 
  * when the instance fits, else the grid form, 2: the grid form.  Both forms
  * need the slot-1 push layout (edge arrays within twice the L2 size).
  * REFORM_PRAQ_MEGA=0|1 in the environment sets the mode at creation.
- * *active (may be NULL) receives the form later runs take: 0 the graph, 1 the
- * grid form, 2 the single-CTA form.  Results equal the graph's bit for bit
+ * *active (may be NULL) receives the form later runs take: 1 the grid form, 2
+ * the single-CTA form, 0 neither.  Results equal the graph's bit for bit
  * (the same tile functions, tile shapes and sums).  Every grid-barrier wait is
  * bounded (1 s of device time): one that runs out ends the launch and the run
  * returns PRAQ_ERROR_CUDA with the context still usable. */

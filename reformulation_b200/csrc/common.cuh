@@ -59,21 +59,23 @@ __device__ __forceinline__ void block_sums(double (&v)[K], double* scratch, doub
 }
 
 // Deterministic sum of `count` rows of K doubles (row-major, stride K) by one
-// block: thread t adds rows t, t + blockDim, ... in order, then block_sums.
+// block: thread t < `threads` adds rows t, t + threads, ... in order, then
+// block_sums (a thread beyond `threads` adds nothing, which leaves every sum's
+// bits as they are, so a wider block gives a narrower one's result).
 // A thread's rows are loaded four at a time by predicated loads, so each
 // group of four costs one memory round trip.
 template <int K>
 __device__ __forceinline__ void reduce_rows(const double* rows, int count, double* scratch,
-                                            double* out) {
+                                            double* out, int threads) {
     constexpr int kRows = 4;
     double v[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) v[k] = 0.0;
-    for (int r0 = threadIdx.x; r0 < count; r0 += kRows * blockDim.x) {
+    for (int r0 = int(threadIdx.x) < threads ? int(threadIdx.x) : count; r0 < count; r0 += kRows * threads) {
         double t[kRows][K];
 #pragma unroll
         for (int u = 0; u < kRows; ++u) {
-            const int r = r0 + u * int(blockDim.x);
+            const int r = r0 + u * threads;
             if (r < count) {
 #pragma unroll
                 for (int k = 0; k < K; ++k) t[u][k] = rows[size_t(r) * K + k];
@@ -81,13 +83,18 @@ __device__ __forceinline__ void reduce_rows(const double* rows, int count, doubl
         }
 #pragma unroll
         for (int u = 0; u < kRows; ++u) {
-            if (r0 + u * int(blockDim.x) < count) {
+            if (r0 + u * threads < count) {
 #pragma unroll
                 for (int k = 0; k < K; ++k) v[k] += t[u][k];
             }
         }
     }
     block_sums<K>(v, scratch, out);
+}
+
+template <int K>
+__device__ __forceinline__ void reduce_rows(const double* rows, int count, double* scratch, double* out) {
+    reduce_rows<K>(rows, count, scratch, out, int(blockDim.x));
 }
 
 // Programmatic dependent launch: a kernel launched with the programmatic

@@ -562,9 +562,10 @@ __device__ __forceinline__ void check_body(Control* c, Params p, const double* s
     if (mode == 2 && !c->restart) return;
     __shared__ double scratch[kEdgeSums * 32];
     __shared__ double node[kNodeSums], edge[kEdgeSums], low[1];
-    reduce_rows<kNodeSums>(pnode, nbn, scratch, node);
-    reduce_rows<kEdgeSums>(pedge, nbe, scratch, edge);
-    if (mode != 2) reduce_rows<1>(plower, nbl, scratch, low);
+    // (the order of kCheckBlock threads, whatever the block)
+    reduce_rows<kNodeSums>(pnode, nbn, scratch, node, kCheckBlock);
+    reduce_rows<kEdgeSums>(pedge, nbe, scratch, edge, kCheckBlock);
+    if (mode != 2) reduce_rows<1>(plower, nbl, scratch, low, kCheckBlock);
     if (threadIdx.x != 0) return;
     if (mode == 2) {
         c->fp_error = canonical(node, edge, c->omega);
@@ -832,23 +833,33 @@ __device__ __forceinline__ void part_sums(const double (&v)[K], double* scratch,
     __syncthreads();
 }
 
-// A run of `v` added in order from zero.
+// A run of `v` added in order from zero, eight loads in flight (a value past
+// the end adds zero, which changes no sum's bits).
 template <class Acc, class Real>
 __device__ __forceinline__ Acc tiny_run(const int* ptr, const Real* v, int i, int m, int* status) {
+    constexpr int U = 8;
     Acc s = Acc(0);
     const int k0 = ptr[i], e = ptr[i + 1];
     if (!index_ok(0 <= k0 && k0 <= e && e <= m, status)) return s;
-    for (int k = k0; k < e; ++k) s += Acc(v[k]);
+    for (int k = k0; k < e; k += U) {
+        Real t[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) t[u] = v[min(k + u, e - 1)];
+#pragma unroll
+        for (int u = 0; u < U; ++u) s += k + u < e ? Acc(t[u]) : Acc(0);
+    }
     return s;
 }
 
-// node_kernel_tile's step, term for term, one thread per node.
+// node_kernel_tile's step, term for term, one thread per node; the node tiles
+// kTinyParts at a time, dealt round-robin to the grid's CTAs (one in the
+// single-CTA form, the cluster's in the cluster form).
 template <class Real, bool Reflect, bool Check>
 __device__ __forceinline__ void tiny_node(const Dev<Real>& d, const Real* ys, const Real* yc, int step, int bounds_at_1,
                                           int gate, int nb_node, double* scratch, double* qout) {
     const Control* c = d.ctl;
     if (skip(c, gate)) return;
-    for (int base = 0; base < nb_node * kBlock; base += kTinyThreads) {
+    for (int base = int(blockIdx.x) * kTinyThreads; base < nb_node * kBlock; base += int(gridDim.x) * kTinyThreads) {
         const int i = base + int(threadIdx.x);
         double acc[kNodeSums] = {0.0, 0.0, 0.0};
         if (i < d.n) {
@@ -892,7 +903,8 @@ __device__ __forceinline__ void tiny_node(const Dev<Real>& d, const Real* ys, co
     }
 }
 
-// edge_kernel_tile's step, term for term, the tiles two at a time.
+// edge_kernel_tile's step, term for term, the tiles two at a time, dealt as
+// tiny_node's.
 template <class Real, bool Reflect, bool Check>
 __device__ __forceinline__ void tiny_edge(const Dev<Real>& d, const Real* ysrc, int step, int bounds_at_1, int gate,
                                           int nb_edge, double* scratch, double* qout) {
@@ -902,7 +914,7 @@ __device__ __forceinline__ void tiny_edge(const Dev<Real>& d, const Real* ysrc, 
     const double kn = Reflect ? double(c->restart_iter + step + 2) : 1.0;
     const Real lwn = Real(kn / (kn + 1.0)), rwn = Real(1.0 / (kn + 1.0));
     const int q = int(threadIdx.x >> 8), t = int(threadIdx.x & (kBlock - 1));
-    for (int tile0 = 0; tile0 < nb_edge; tile0 += kTinyParts) {
+    for (int tile0 = int(blockIdx.x) * kTinyParts; tile0 < nb_edge; tile0 += int(gridDim.x) * kTinyParts) {
         const int tile = tile0 + q;
         const int base = tile * (kBlock * kEdgesPerThread) + t;
         double acc[kEdgeSums] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -960,7 +972,7 @@ template <class Real>
 __device__ __forceinline__ void tiny_lower(const Dev<Real>& d, const Real* ys, const Real* yc, int nb_node,
                                            double* scratch, double* qout) {
     if (d.ctl->terminated) return;
-    for (int base = 0; base < nb_node * kBlock; base += kTinyThreads) {
+    for (int base = int(blockIdx.x) * kTinyThreads; base < nb_node * kBlock; base += int(gridDim.x) * kTinyThreads) {
         const int i = base + int(threadIdx.x);
         double acc[1] = {0.0};
         if (i < d.n) {
@@ -1229,6 +1241,290 @@ tiny_solve_kernel(const __grid_constant__ Dev<Real> g, const __grid_constant__ P
     if (threadIdx.x == 0) *g.ctl = *d.ctl;
 }
 
+// ---- the whole solve in one cluster's shared memory ------------------------
+// Above one CTA's shared memory and up to some ten thousand edges, a step on
+// the graph is two kernels of a few microseconds each that hold a microsecond
+// of work.  cluster_solve_kernel runs the solve in ONE thread-block cluster of
+// up to kClusterMax CTAs of kTinyThreads, the instance spread over their
+// shared memories:
+// * a CTA owns a range of nodes (cut so that the bytes balance), the first-end
+//   edges of those nodes (one range of the sorted edges) and their slot-1
+//   values (one range of second-end order);
+// * every CTA holds a copy of the whole reflection r, written by the nodes'
+//   owners to all of them through distributed shared memory, so the edge half
+//   gathers from its own shared memory;
+// * an edge's slot-1 value goes straight to the shared memory of its second
+//   end's owner (its address there is worked out once a launch), so a node
+//   adds both its runs from its own.
+// A plain step is two cluster barriers (a few hundred cycles each, against the
+// 2,500 of a grid barrier through L2) and touches no global memory.  The steps
+// with check sums, the bounds, the check and the restart step run the
+// single-CTA form's code over the graph's tiles in global memory, to which the
+// iterates are written back before them.  Arithmetic and sums are the graph's
+// term for term, so the results are the graph's bit for bit.
+constexpr int kClusterMax = 16;
+
+// The cut of an instance over a cluster: nodes, sorted edges and second-end
+// positions of CTA q are [node[q], node[q + 1]) and so on.
+struct ClusterPlan {
+    int node[kClusterMax + 1], edge[kClusterMax + 1], second[kClusterMax + 1];
+    int max_nodes, max_edges, max_seconds;
+};
+static_assert(sizeof(ClusterPlan) <= 256, "read back through a pinned mirror slot");
+
+// Bytes a node, a first-end edge and a slot-1 value take in their CTA.
+__host__ __device__ inline int cluster_node_bytes(int real) { return 5 * real + 8; }
+__host__ __device__ inline int cluster_edge_bytes(int real) { return 12 + 3 * real; }
+
+struct ClusterLayout {
+    size_t r, x1, x2, x0, diag, deg, rp, cp, pred, pred1, u0, w, ends, dst, total;
+};
+__host__ __device__ inline ClusterLayout cluster_layout(int n, int nodes, int edges, int seconds, int real) {
+    ClusterLayout t{};
+    size_t at = 0;
+    t.r = tiny_take(at, size_t(n + 3) / 4 * 4 * real);   // whole vectors
+    t.x1 = tiny_take(at, size_t(nodes) * real);
+    t.x2 = tiny_take(at, size_t(nodes) * real);
+    t.x0 = tiny_take(at, size_t(nodes) * real);
+    t.diag = tiny_take(at, size_t(nodes) * real);
+    t.deg = tiny_take(at, size_t(nodes) * real);
+    t.rp = tiny_take(at, size_t(nodes + 1) * sizeof(int));
+    t.cp = tiny_take(at, size_t(nodes + 1) * sizeof(int));
+    t.pred = tiny_take(at, size_t(edges) * real);
+    t.pred1 = tiny_take(at, size_t(seconds) * real);
+    t.u0 = tiny_take(at, size_t(edges) * real);
+    t.w = tiny_take(at, size_t(edges) * real);
+    t.ends = tiny_take(at, size_t(edges) * sizeof(int2));
+    t.dst = tiny_take(at, size_t(edges) * sizeof(unsigned));
+    t.total = at;
+    return t;
+}
+
+// Cut q of `parts`: the first node at which the bytes before it (a monotone
+// sum of run pointers) reach q shares of the total.
+__global__ void cluster_plan_kernel(int n, int m, int parts, int real, const int* __restrict__ row_ptr,
+                                    const int* __restrict__ col_ptr, ClusterPlan* plan) {
+    __shared__ int node[kClusterMax + 1];
+    const int q = threadIdx.x;
+    auto bytes = [&](int i) {
+        return (long long)cluster_edge_bytes(real) * row_ptr[i] + (long long)real * col_ptr[i] +
+               (long long)cluster_node_bytes(real) * i;
+    };
+    if (q <= parts) {
+        const long long want = bytes(n) * q / parts;
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (bytes(mid) < want) lo = mid + 1; else hi = mid;
+        }
+        node[q] = q == parts ? n : lo & ~3;   // a CTA's part of r starts on 16 bytes
+    }
+    __syncthreads();
+    if (q <= kClusterMax) {   // cuts past `parts` are empty
+        const int i = node[min(q, parts)];
+        plan->node[q] = i;
+        plan->edge[q] = row_ptr[i];
+        plan->second[q] = col_ptr[i];
+    }
+    if (q == 0) {
+        int a = 0, b = 0, c = 0;
+        for (int k = 0; k < parts; ++k) {
+            a = max(a, node[k + 1] - node[k]);
+            b = max(b, row_ptr[node[k + 1]] - row_ptr[node[k]]);
+            c = max(c, col_ptr[node[k + 1]] - col_ptr[node[k]]);
+        }
+        plan->max_nodes = a;
+        plan->max_edges = b;
+        plan->max_seconds = c;
+    }
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_address(unsigned own, int rank) {   // the same place in CTA `rank`
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(own), "r"(rank));
+    return a;
+}
+// 16 bytes at `own` of this CTA to the same place in CTA `rank`
+__device__ __forceinline__ void copy_cluster_vec(unsigned own, int rank) {
+    unsigned a, b, c, e;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(e) : "r"(own) : "memory");
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_address(own, rank)), "r"(a), "r"(b),
+                 "r"(c), "r"(e)
+                 : "memory");
+}
+__device__ __forceinline__ void store_cluster(unsigned at, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+}
+__device__ __forceinline__ void store_cluster(unsigned at, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+
+template <class Real>
+__global__ void __launch_bounds__(kTinyThreads, 1)
+cluster_solve_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant__ Params prm,
+                     const ClusterPlan* __restrict__ plan, int nb_node, int nb_edge, int max_nodes, int max_edges,
+                     int max_seconds, int start, int max_blocks) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double scratch[kTinyParts * kEdgeSums * 32];
+    __shared__ double qout[kTinyParts * kEdgeSums];
+    __shared__ StepWeights<Real> weights[kStepTable];
+    __shared__ int second_cut[kClusterMax + 1];
+    const int parts = int(gridDim.x), rank = int(blockIdx.x), tid = int(threadIdx.x);   // one cluster: the grid
+    const ClusterLayout L = cluster_layout(d.n, max_nodes, max_edges, max_seconds, int(sizeof(Real)));
+    const int n0 = plan->node[rank], nodes = plan->node[rank + 1] - n0;
+    const int e0 = plan->edge[rank], edges = plan->edge[rank + 1] - e0;
+    const int k0 = plan->second[rank], seconds = plan->second[rank + 1] - k0;
+    auto reals = [&](size_t off) { return reinterpret_cast<Real*>(smem_raw + off); };
+    Real* const r = reals(L.r);
+    Real* const x1 = reals(L.x1);
+    Real* const x2 = reals(L.x2);
+    Real* const x0 = reals(L.x0);
+    Real* const diag = reals(L.diag);
+    Real* const deg = reals(L.deg);
+    Real* const pred = reals(L.pred);
+    Real* const pred1 = reals(L.pred1);
+    Real* const u0 = reals(L.u0);
+    Real* const w = reals(L.w);
+    int* const rp = reinterpret_cast<int*>(smem_raw + L.rp);
+    int* const cp = reinterpret_cast<int*>(smem_raw + L.cp);
+    int2* const ends = reinterpret_cast<int2*>(smem_raw + L.ends);
+    unsigned* const dst = reinterpret_cast<unsigned*>(smem_raw + L.dst);
+    if (tid <= kClusterMax) second_cut[tid] = plan->second[tid];
+    __syncthreads();
+    for (int i = tid; i < nodes; i += kTinyThreads) {
+        diag[i] = d.diag[n0 + i];
+        deg[i] = d.deg[n0 + i];
+    }
+    for (int i = tid; i <= nodes; i += kTinyThreads) {
+        rp[i] = d.row_ptr[n0 + i] - e0;
+        cp[i] = d.col_ptr[n0 + i] - k0;
+    }
+    const unsigned pred1_at = shared_address(pred1), r_at = shared_address(r);
+    for (int e = tid; e < edges; e += kTinyThreads) {
+        const int2 ij = d.ends[e0 + e];
+        int pos = d.colpos[e0 + e];
+        if (!index_ok(unsigned(ij.x) < unsigned(d.n) && unsigned(ij.y) < unsigned(d.n) && unsigned(pos) < unsigned(d.m),
+                      &d.ctl->status))
+            pos = 0;
+        int q = 0;   // the CTA whose nodes this second-end position belongs to
+        while (q + 1 < parts && pos >= second_cut[q + 1]) ++q;
+        ends[e] = index_ok(unsigned(ij.x) < unsigned(d.n) && unsigned(ij.y) < unsigned(d.n), &d.ctl->status)
+                      ? ij : make_int2(0, 0);
+        w[e] = d.w[e0 + e];
+        dst[e] = cluster_address(pred1_at, q) + unsigned(pos - second_cut[q]) * unsigned(sizeof(Real));
+    }
+    auto check = [&](int mode) {
+        if (rank == 0) tiny_check(d.ctl, prm, d.scale, d.pnode, nb_node, d.pedge, nb_edge, d.plower, mode);
+        cluster_barrier();
+    };
+    if (start) {   // the start step with the bounds at the start point, and the check before the loop
+        tiny_node<Real, false, true>(d, d.pred, d.pred1, 0, 1, 0, nb_node, scratch, qout);
+        tiny_lower<Real>(d, d.pred, d.pred1, nb_node, scratch, qout);
+        cluster_barrier();
+        tiny_edge<Real, false, true>(d, d.pred, 0, 1, 0, nb_edge, scratch, qout);
+        cluster_barrier();
+        check(0);
+    }
+    const int op = int(prm.op_steps);
+    for (int b = 0; b < max_blocks; ++b) {
+        const Control* c = d.ctl;
+        if (c->terminated) break;   // uniform over the cluster: the check is the last writer
+        const double omega = c->omega;
+        const long long since = c->restart_iter;
+        const Real ps = Real(kEta / omega), hs = Real(0.5 * kEta * omega);
+        // the iterates as the last block left them
+        for (int i = tid; i < nodes; i += kTinyThreads) {
+            x1[i] = d.x1[n0 + i];
+            x2[i] = d.x2[n0 + i];
+            x0[i] = d.x0[n0 + i];
+        }
+        for (int e = tid; e < edges; e += kTinyThreads) {
+            pred[e] = d.pred[e0 + e];
+            u0[e] = d.u0[e0 + e];
+        }
+        for (int k = tid; k < seconds; k += kTinyThreads) pred1[k] = d.pred1[k0 + k];
+        for (int s = 0; s + 1 < op; ++s) {
+            if (s % kStepTable == 0) {
+                __syncthreads();
+                if (tid < kStepTable) weights[tid] = step_weights<Real>(since, s + tid);
+                cluster_barrier();   // (s = 0: every CTA holds the block's iterates before a peer writes slot 1)
+            }
+            const StepWeights<Real> sw = weights[s % kStepTable];
+            {   // the node half: two threads a node, a run each
+                const int half = tid & 1;
+                const int* const ptr = half ? cp : rp;
+                const Real* const v = half ? pred1 : pred;
+                for (int base = 0; base < nodes; base += kTinyThreads / 2) {
+                    const int i = base + (tid >> 1);
+                    Real sum = Real(0);
+                    if (i < nodes) sum = shared_run<Real>(v, ptr[i], ptr[i + 1]);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                    if (i < nodes) {   // (both threads of the pair compute it; one stores the point)
+                        const Real x2o = x2[i], x1v = rfma(sw.lw, rfma(Real(2), x2o, -x1[i]), rmul(sw.rw, x0[i]));
+                        const Real x2v = clampv(rfma(-ps, (diag[i] - sum) / deg[i], x1v), Real(0), Real(1));
+                        const Real rv = rfma(Real(2), x2v, -x1v);
+                        __syncwarp(3u << (tid & 30));   // the pair has read the point before one stores it
+                        if (!half) {
+                            x1[i] = x1v;
+                            x2[i] = x2v;
+                            r[n0 + i] = rv;
+                        }
+                    }
+                }
+                // this CTA's part of r to every other, 16 bytes a store
+                __syncthreads();
+                const int vecs = (nodes * int(sizeof(Real)) + 15) / 16;
+                const unsigned mine = r_at + unsigned(n0) * unsigned(sizeof(Real));
+                for (int k = tid; k < vecs * (parts - 1); k += kTinyThreads) {
+                    const int p = k / vecs, v = k - p * vecs;
+                    copy_cluster_vec(mine + 16u * unsigned(v), p + (p >= rank ? 1 : 0));
+                }
+            }
+            cluster_barrier();
+#pragma unroll 2
+            for (int e = tid; e < edges; e += kTinyThreads) {   // the edge half
+                const int2 ij = ends[e];
+                const Real wv = w[e], u1 = pred[e], ua = u0[e];
+                const unsigned to = dst[e];
+                const Real ri = r[ij.x], rj = r[ij.y];
+                const bool cov = wv > Real(0);
+                const Real wa = cov ? wv : -wv;
+                const Real u2 = cov ? clampv(rfma(hs, (Real(1) - ri) - rj, u1), -wa, Real(0))
+                                    : clampv(rfma(hs, rj - ri, u1), Real(0), wa);
+                const Real nx = rfma(sw.lwn, rfma(Real(2), u2, -u1), rmul(sw.rwn, ua));
+                pred[e] = nx;
+                store_cluster(to, cov ? nx : wa - nx);
+            }
+            cluster_barrier();
+        }
+        // back to global memory, where the rest of the block runs
+        for (int i = tid; i < nodes; i += kTinyThreads) {
+            d.x1[n0 + i] = x1[i];
+            d.x2[n0 + i] = x2[i];
+        }
+        for (int e = tid; e < edges; e += kTinyThreads) d.pred[e0 + e] = pred[e];
+        for (int k = tid; k < seconds; k += kTinyThreads) d.pred1[k0 + k] = pred1[k];
+        cluster_barrier();
+        tiny_node<Real, true, true>(d, d.pred, d.pred1, op - 1, 0, 0, nb_node, scratch, qout);
+        cluster_barrier();
+        tiny_edge<Real, true, true>(d, nullptr, op - 1, 0, 0, nb_edge, scratch, qout);
+        cluster_barrier();
+        tiny_lower<Real>(d, d.u2s, d.u2s1, nb_node, scratch, qout);
+        cluster_barrier();
+        check(1);
+        if (d.ctl->restart) {   // uniform over the cluster
+            tiny_node<Real, false, true>(d, d.u2s, d.u2s1, 0, 0, 1, nb_node, scratch, qout);
+            cluster_barrier();
+            tiny_edge<Real, false, true>(d, d.u2s, 0, 0, 1, nb_edge, scratch, qout);
+            cluster_barrier();
+            check(2);
+        }
+    }
+}
+
 // Cold start: the centroid, x = 1/2 and y_e = (-W_ij, -W_ij) / scale, which is
 // u = -w / 2 in the one-coordinate form (half_edge.py:87-94).
 template <class Real>
@@ -1469,6 +1765,13 @@ struct Solver final : SolverBase {
     bool tiny = false, tiny_fits = false;
     size_t tiny_smem = 0;
     static constexpr int kTinyBlocks = 128;
+    // The cluster form (cluster_solve_kernel): CTAs of its cluster (0: the
+    // instance does not take it), its cut and dynamic shared memory.
+    bool clustered = false;
+    int cluster_ctas = 0;
+    size_t cluster_smem = 0;
+    PoolBuf<ClusterPlan> plan;
+    ClusterPlan hplan{};
 
     ~Solver() override {
         if (stream) cudaStreamSynchronize(stream);
@@ -1483,6 +1786,7 @@ struct Solver final : SolverBase {
         u0.release(); u2s.release(); u2s1.release();
         pnode.release(); pedge.release(); plower.release(); scale.release(); ctl.release(); bar.release();
         trace.release();
+        plan.release();
         warm_x.release(); warm_y.release();
         if (stream) cudaStreamSynchronize(stream);
         pinned_put(mirror);
@@ -1592,6 +1896,7 @@ struct Solver final : SolverBase {
             tiny_smem = tiny_layout(n, m, nb_node, nb_edge, int(sizeof(Real))).total;
             // check_body's row reductions keep the 256-thread order up to 256 rows
             tiny_fits = tiny_smem <= size_t(room) && nb_node <= kBlock && nb_edge <= kBlock;
+            if (!tiny_fits) RB_CUDA_TRY(init_cluster());
         }
         // REFORM_PRAQ_MEGA=0|1 sets the initial mode (tests, measurements);
         // REFORM_PRAQ_MEGA_PHANTOM=k makes every barrier wait for k CTAs that
@@ -1607,6 +1912,93 @@ struct Solver final : SolverBase {
         return set_mega(mode);
     }
 
+    // CTAs of the largest cluster of cluster_solve_kernel the device can hold at
+    // once with all of an SM's shared memory each (0: none), and that memory.
+    static cudaError_t cluster_limits(int* ctas, int* room) {
+        RB_CUDA_TRY(once_per_device(room, [](int* v) {
+            int dev = 0, optin = 0;
+            cudaFuncAttributes fa{};
+            RB_CUDA_TRY(cudaGetDevice(&dev));
+            RB_CUDA_TRY(cudaFuncGetAttributes(&fa, cluster_solve_kernel<Real>));
+            RB_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+            *v = optin > int(fa.sharedSizeBytes) ? optin - int(fa.sharedSizeBytes) : 0;
+            RB_CUDA_TRY(cudaFuncSetAttribute(cluster_solve_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, *v));
+            return cudaFuncSetAttribute(cluster_solve_kernel<Real>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        }));
+        const int bytes = *room;
+        return once_per_device(ctas, [bytes](int* v) {
+            *v = 0;
+            for (int c = kClusterMax; c >= 2 && !*v; c >>= 1) {
+                cudaLaunchConfig_t cfg = {};
+                cudaLaunchAttribute attr[1];
+                cluster_config(cfg, attr, c, size_t(bytes), nullptr);
+                int held = 0;
+                if (cudaOccupancyMaxActiveClusters(&held, cluster_solve_kernel<Real>, &cfg) == cudaSuccess && held > 0)
+                    *v = c;
+            }
+            (void)cudaGetLastError();
+            return cudaSuccess;
+        });
+    }
+
+    static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int ctas, size_t smem, cudaStream_t st) {
+        cfg.gridDim = dim3(unsigned(ctas));
+        cfg.blockDim = dim3(unsigned(kTinyThreads));
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = unsigned(ctas);
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+
+    // A step of the cluster form costs its remote stores (r to 15 CTAs, a
+    // slot-1 value an edge); the graph's costs its launches.  Per solve, graph
+    // against cluster, FP32 / FP64: n = 700, m = 3,500 - / 0.65 against 0.36 ms;
+    // 1,000, 6,000 0.66 against 0.48 / 0.84 against 0.50; 2,000, 10,000 0.53
+    // against 0.46 / 0.68 against 0.45; 3,000, 12,000 0.64 against 0.63 / 0.80
+    // against 0.68; 3,000, 24,000 0.58 against 0.64 / 0.74 against 0.70; 5,000,
+    // 30,000 0.69 against 0.97 / 0.88 against 1.10.  (8 CTAs were slower than
+    // 16 from n = 1,500 up.)
+    static constexpr int kClusterNodes = sizeof(Real) == 4 ? 2048 : 3072;
+    static constexpr int kClusterEdges = sizeof(Real) == 4 ? 12288 : 24576;
+
+    // Cut the instance over a cluster, if its bytes can fit one: the cut is
+    // made on the device (it needs the run pointers) and read back.
+    cudaError_t init_cluster() {
+        cluster_ctas = 0;
+        const char* env = std::getenv("REFORM_PRAQ_CLUSTER");   // 0: never (tests, measurements)
+        if (m == 0 || (env && !std::strcmp(env, "0"))) return cudaSuccess;
+        if (n > kClusterNodes || m > kClusterEdges) return cudaSuccess;
+        int ctas = 0, room = 0;
+        RB_CUDA_TRY(cluster_limits(&ctas, &room));
+        const int real = int(sizeof(Real));
+        const double share = (double(m) * (cluster_edge_bytes(real) + real) + double(n) * cluster_node_bytes(real)) /
+                             std::max(ctas, 1);
+        if (ctas < 2 || share + double(n) * real > double(room)) return cudaSuccess;   // no cut can fit
+        RB_CUDA_TRY(plan.alloc(1, stream));
+        cluster_plan_kernel<<<1, 32, 0, stream>>>(n, m, ctas, real, row_ptr.ptr, col_ptr.ptr, plan.ptr);
+        RB_CUDA_TRY(cudaMemcpyAsync(mirror, plan.ptr, sizeof(ClusterPlan), cudaMemcpyDeviceToHost, stream));
+        RB_CUDA_TRY(cudaStreamSynchronize(stream));
+        std::memcpy(&hplan, mirror, sizeof(ClusterPlan));
+        std::memset(static_cast<void*>(mirror), 0, sizeof(Control));   // no run yet
+        cluster_smem = cluster_layout(n, hplan.max_nodes, hplan.max_edges, hplan.max_seconds, real).total;
+        if (cluster_smem <= size_t(room)) cluster_ctas = ctas;
+        return cudaSuccess;
+    }
+
+    cudaError_t launch_cluster(int start) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        cluster_config(cfg, attr, cluster_ctas, cluster_smem, stream);
+        // a wall-clock budget is looked at between launches: one block in each then
+        return cudaLaunchKernelEx(&cfg, cluster_solve_kernel<Real>, d, prm, (const ClusterPlan*)plan.ptr, nb_node, nb_edge,
+                                  hplan.max_nodes, hplan.max_edges, hplan.max_seconds, start,
+                                  time_limit >= 0.0 ? 1 : kTinyBlocks);
+    }
+
     // mode -1: automatic (the single-CTA form wherever the instance fits one
     // CTA's shared memory, else the graph: per solve 0.21 against 0.60 ms at
     // n = 200, m = 1,000, 0.36 against 0.64 at n = 700, m = 2,800, 1.63 against
@@ -1617,6 +2009,7 @@ struct Solver final : SolverBase {
     cudaError_t set_mega(int mode) {
         mega_mode = mode < 0 ? -1 : (mode > 2 ? 2 : mode);
         tiny = tiny_fits && (mega_mode == 1 || mega_mode == -1);
+        clustered = !tiny && mega_mode == -1 && cluster_ctas > 0;
         mega = !tiny && mega_mode >= 1 && mega_grid > 0;
         if (mega && !bar.ptr) {
             RB_CUDA_TRY(bar.alloc(1, stream));
@@ -1640,7 +2033,7 @@ struct Solver final : SolverBase {
         return cudaLaunchKernelEx(&cfg, tiny_solve_kernel<Real>, d, prm, nb_node, nb_edge, start, kTinyBlocks);
     }
 
-    // A solve in the single-CTA form: the start point set in global memory,
+    // A solve in the single-CTA or the cluster form: the start point set in global memory,
     // then launches of up to kTinyBlocks check blocks (the first with the
     // start step and its check) until the solve ends; the wall-clock budget
     // is checked between launches.
@@ -1655,7 +2048,8 @@ struct Solver final : SolverBase {
         nlaunch += 1;
         bool timed_out = false;
         for (int first = 1;; first = 0) {
-            if (mark_begin(9) != cudaSuccess || launch_tiny(first) != cudaSuccess || mark_end() != cudaSuccess)
+            if (mark_begin(9) != cudaSuccess || (tiny ? launch_tiny(first) : launch_cluster(first)) != cudaSuccess ||
+                mark_end() != cudaSuccess)
                 return PRAQ_ERROR_CUDA;
             nlaunch += 1;
             if (cudaMemcpyAsync(mirror, d.ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
@@ -1973,7 +2367,7 @@ struct Solver final : SolverBase {
 
     int run() override {
         const auto started = std::chrono::steady_clock::now();
-        if (tiny) return run_tiny(started);
+        if (tiny || clustered) return run_tiny(started);
         bool timed_out = false;
         // the first run launches directly; repeated runs replay a captured block
         if (runs++ > 0 && !exec && !mega && capture_block() != cudaSuccess) return PRAQ_ERROR_CUDA;
@@ -2026,7 +2420,7 @@ struct Solver final : SolverBase {
     // block.
     int run_profiled(double* ms, long long* count) override {
         for (int k = 0; k < kKinds; ++k) { ms[k] = 0.0; count[k] = 0; }
-        if (tiny) {   // each launch of the single-CTA form as one mark of kind 9
+        if (tiny || clustered) {   // each launch of either form as one mark of kind 9
             marks.clear();
             profiling = true;
             const double budget = time_limit;

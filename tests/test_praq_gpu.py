@@ -506,6 +506,40 @@ def test_single_cta_plain_steps_equal_graph(native, use_float32, n, m, op_steps)
     assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
 
 
+@pytest.mark.parametrize("use_float32", [0, 1])
+@pytest.mark.parametrize("case", ["small", "odd", "hub", "few-nodes", "largest", "long-block"])
+def test_cluster_form_equals_graph(native, use_float32, case):
+    """The automatic choice between one CTA's shared memory and the graph, a
+    solve in one cluster's shared memory, against the graph bit for bit: just
+    above the single-CTA form, odd sizes, a hub whose run is most of the edges
+    (an uneven cut), fewer nodes than threads in the cluster, the largest sizes
+    it takes, and a block of more steps than the weights' table.  Cold and warm
+    starts; two launches a solve show that the form was taken."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import Library
+    op = 130 if case == "long-block" else 16
+    if case == "hub":
+        n, rng = 2000, np.random.default_rng(2)
+        rest = qubo_uniform_edges(3, n, 4000)
+        rows = np.concatenate([np.zeros(n - 1, np.int64), rest.rows[rest.rows > 0]])
+        cols = np.concatenate([np.arange(1, n), rest.cols[rest.rows > 0]])
+        inst = QuboInstance("hub", "hub", n, rest.diag, rows, cols, rng.integers(1, 100, rows.size) * 1.0)
+    else:
+        n, m = {"small": (900, 6000), "odd": (1237, 7001), "few-nodes": (130, 7000), "long-block": (901, 6001),
+                "largest": (2048, 12288) if use_float32 else (3072, 24576)}[case]
+        inst = qubo_uniform_edges(7, n, m)
+    p = Library().parameters(tolerance=1e-4 if use_float32 else 1e-7, use_float32=use_float32, max_iter=2080,
+                             op_steps=op)
+    rng = np.random.default_rng(1)
+    warm = (rng.uniform(0, 1, inst.n), rng.normal(0, 5, (inst.edges, 2)))
+    _, auto, launches = _praq_runs(inst, p, -1, warm=warm)
+    _, graph, _ = _praq_runs(inst, p, 0, warm=warm)
+    assert launches == 2
+    for (a, ya), (b, yb) in zip(auto, graph):
+        assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
+        assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
+
+
 def test_persistent_kernel_choice_and_edgeless(native):
     from reformulation_b200.instances import qubo_uniform_edges
     from reformulation_b200.praq import DeviceSolver, Library
