@@ -156,30 +156,59 @@ constexpr int kPull = RB200_PRAQ_PULL;
 template <class Real>
 constexpr int stage_len() { return RB200_PRAQ_STAGE_BYTES / int(sizeof(Real)); }
 
-// The sums of v over the runs [ptr[i], ptr[i+1]) of the 32 consecutive nodes
-// i = base + lane of a warp, one node per lane.  The runs of consecutive nodes
-// are adjacent, so the warp copies the whole range [ptr[base], ptr[base+32])
-// through shared memory in coalesced passes of kStage values, and each lane
+// What a kernel of a programmatic chain does between what it may read at once
+// and what the kernel ahead of it writes: wait for that kernel, then let the
+// next one start.  A kernel that has started found every kernel before its
+// predecessor complete (the predecessor waited for them before it let this one
+// start), so before the wait it may read the instance's constants and whatever
+// its predecessor does not write; the latency of those loads then runs beside
+// the predecessor's last CTAs.  (Waiting first and then reading everything:
+// n = 3,000, m = 24,000 0.56 against 0.51 ms a solve in FP32, 0.74 against 0.65
+// in FP64; 50,000, 200,000 FP64 1.16 against 1.00; 1e5, 1e6 1.41 against 1.35
+// and 1.71 against 1.64; 2e6, 2e7 26.6 against 26.4.)  NoWait: everything is
+// there (persistent kernels, the batched engine).
+struct NoWait {
+    __device__ __forceinline__ void operator()() const {}
+};
+struct PdlWait {
+    __device__ __forceinline__ void operator()() const {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
+};
+
+// The runs of a warp's 32 consecutive nodes base + lane: the warp's whole
+// range [lo, hi) and this lane's own [a, b) (empty past the last node).
+struct RunBounds {
+    int lo = 0, hi = 0, a = 0, b = 0;
+};
+__device__ __forceinline__ RunBounds run_bounds(const int* __restrict__ ptr, int n, long long base, int lane) {
+    RunBounds r;
+    if (base >= n) return r;   // uniform over the warp
+    const long long i = base + lane;
+    r.lo = ptr[base];
+    r.hi = ptr[base + 32 < n ? base + 32 : n];
+    if (i < n) {
+        r.a = ptr[i];
+        r.b = ptr[i + 1];
+    }
+    return r;
+}
+
+// The sums of v over the runs `run` of the 32 consecutive nodes of a warp, one
+// node per lane.  The runs of consecutive nodes are adjacent, so the warp
+// copies their whole range through shared memory in coalesced passes of kStage values, and each lane
 // adds its own run's part of every pass in order.  All lanes of the warp must
 // call it (with the same base).  Few registers: the form for grids of many
 // waves, where the issue rate, not the latency of one warp, bounds the kernel
 // (chunks of 4 loads per lane: 2 % faster per solve at n >= 1.5e5 than an
 // unrolled loop; 8 were no better).
 template <class Real, class Acc, bool Indexed>
-__device__ __forceinline__ Acc warp_runs(const int* __restrict__ ptr, const Real* v, const int* __restrict__ idx,
-                                         int n, long long base, int lane, Real* __restrict__ stage, int m,
-                                         int* status) {
-    if (base >= n) return Acc(0);   // uniform over the warp
-    const long long i = base + lane;
-    const long long last = base + 32 < n ? base + 32 : n;
-    const int lo_all = ptr[base], hi_all = ptr[last];
+__device__ __forceinline__ Acc warp_runs(const RunBounds& run, const Real* v, const int* __restrict__ idx, int lane,
+                                         Real* __restrict__ stage, int m, int* status) {
+    const int lo_all = run.lo, hi_all = run.hi, a = run.a, b = run.b;
     // the warp's range, the same on every lane (the runs inside it follow)
     if (!index_ok(0 <= lo_all && lo_all <= hi_all && hi_all <= m, status)) return Acc(0);
-    int a = 0, b = 0;
-    if (i < n) {
-        a = ptr[i];
-        b = ptr[i + 1];
-    }
     constexpr int kStage = stage_len<Real>();
     Acc s = Acc(0);
     for (int c0 = lo_all; c0 < hi_all; c0 += kStage) {
@@ -222,9 +251,9 @@ __device__ __forceinline__ Acc warp_runs(const int* __restrict__ ptr, const Real
     return s;
 }
 
-// The sums, for the 32 consecutive nodes i = base + lane of a warp (one node
-// per lane), of two runs at once: run a = va[pa[i] .. pa[i+1]) and run b =
-// vb[k] (IndexB: vb[ib[k]]) for k in [pb[i], pb[i+1]).  The warp copies the
+// The sums, for the 32 consecutive nodes of a warp (one node per lane), of two
+// runs at once: run a = va[k] for k in `pa`, and run b = vb[k] (IndexB:
+// vb[ib[k]]) for k in `pb`.  The warp copies the
 // ranges of both runs for its 32 nodes through shared memory in passes of
 // kStage values each (run a and run b, or run b's indices, coalesced; with
 // IndexB run b's values gathered), and every lane adds its own runs' parts of
@@ -236,24 +265,14 @@ __device__ __forceinline__ Acc warp_runs(const int* __restrict__ ptr, const Real
 // latency of a warp's dependent loads bounds.  All lanes of the warp must call
 // it with the same base.
 template <class Real, class Acc, bool IndexB>
-__device__ __forceinline__ void warp_runs2(const int* __restrict__ pa, const Real* va, const int* __restrict__ pb,
-                                           const Real* vb, const int* __restrict__ ib, int n, long long base, int lane,
-                                           Real* __restrict__ sa,
+__device__ __forceinline__ void warp_runs2(const RunBounds& pa, const Real* va, const RunBounds& pb, const Real* vb,
+                                           const int* __restrict__ ib, int lane, Real* __restrict__ sa,
                                            Real* __restrict__ sb, Acc& ra, Acc& rb, int m, int* status) {
     ra = Acc(0);
     rb = Acc(0);
-    if (base >= n) return;   // uniform over the warp
-    const long long i = base + lane;
-    const long long last = base + 32 < n ? base + 32 : n;
-    const int alo = pa[base], ahi = pa[last], blo = pb[base], bhi = pb[last];
+    const int alo = pa.lo, ahi = pa.hi, blo = pb.lo, bhi = pb.hi;
     if (!index_ok(0 <= alo && alo <= ahi && ahi <= m && 0 <= blo && blo <= bhi && bhi <= m, status)) return;
-    int a0 = 0, a1 = 0, b0 = 0, b1 = 0;
-    if (i < n) {
-        a0 = pa[i];
-        a1 = pa[i + 1];
-        b0 = pb[i];
-        b1 = pb[i + 1];
-    }
+    const int a0 = pa.a, a1 = pa.b, b0 = pb.a, b1 = pb.b;
     constexpr int kStage = stage_len<Real>();
     constexpr int kPer = kStage / 32;
     static_assert(kStage % 32 == 0, "a pass is whole warp rows");
@@ -314,7 +333,7 @@ __device__ __forceinline__ void warp_runs2(const int* __restrict__ pa, const Rea
     }
 }
 
-// S^T y at node base + lane: the node's run of `ys` (slot 0, first-end order)
+// S^T y at the warp's node of this lane: the node's run of `ys` (slot 0, first-end order)
 // plus its run of slot-1 values of `yc`: in the push layout `yc` is in
 // second-end order, in the pull layout it is in edge order and read through
 // d.colidx (second-end order).  `stage` holds stage_runs<Wide> * stage_len
@@ -333,16 +352,16 @@ __device__ __forceinline__ Real* warp_stage() {
 }
 
 template <class Real, class Acc, bool Wide, bool Pull>
-__device__ __forceinline__ Acc scatter_at(const Dev<Real>& d, const Real* ys, const Real* yc, long long base,
-                                          int lane, Real* __restrict__ stage) {
+__device__ __forceinline__ Acc scatter_at(const Dev<Real>& d, const RunBounds& first, const RunBounds& second,
+                                          const Real* ys, const Real* yc, int lane, Real* __restrict__ stage) {
     if constexpr (Wide) {
         Acc s0, s1;
-        warp_runs2<Real, Acc, Pull>(d.row_ptr, ys, d.col_ptr, yc, d.colidx, d.n, base, lane, stage,
-                                    stage + stage_len<Real>(), s0, s1, d.m, &d.ctl->status);
+        warp_runs2<Real, Acc, Pull>(first, ys, second, yc, d.colidx, lane, stage, stage + stage_len<Real>(), s0, s1, d.m,
+                                    &d.ctl->status);
         return s0 + s1;
     } else {
-        const Acc s0 = warp_runs<Real, Acc, false>(d.row_ptr, ys, nullptr, d.n, base, lane, stage, d.m, &d.ctl->status);
-        const Acc s1 = warp_runs<Real, Acc, Pull>(d.col_ptr, yc, d.colidx, d.n, base, lane, stage, d.m, &d.ctl->status);
+        const Acc s0 = warp_runs<Real, Acc, false>(first, ys, nullptr, lane, stage, d.m, &d.ctl->status);
+        const Acc s1 = warp_runs<Real, Acc, Pull>(second, yc, d.colidx, lane, stage, d.m, &d.ctl->status);
         return s0 + s1;
     }
 }
@@ -351,18 +370,19 @@ __device__ __forceinline__ Acc scatter_at(const Dev<Real>& d, const Real* ys, co
 // (solver.py:259-267 and 276-292).  Reflect: x1 = lw (2 x2 - x1) + rw x0 with
 // k = restart_iter + step + 1; vanilla: x1 = x2 and the anchor becomes x1.
 // Check: the node sums of this step go to pnode.
-template <class Real, bool Reflect, bool Check, bool Wide = false, bool Pull = false>
+template <class Real, bool Reflect, bool Check, bool Wide = false, bool Pull = false, class Wait = NoWait>
 __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, const Real* ys, const Real* yc, int step,
-                                                 int bounds_at_1, int gate) {
+                                                 int bounds_at_1, int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    if (skip(c, gate)) return;
     __shared__ double scratch[kNodeSums * 32];
     Real* stage = warp_stage<Real, stage_runs<Wide>()>();
     const int lane = threadIdx.x & 31;
     const long long base = (long long)tile * blockDim.x + (threadIdx.x & ~31);
     const long long i = base + lane;
     const bool owner = i < d.n;
-    // node data first, so its latency hides behind the gather
+    // the run bounds and the node data: nothing the kernel ahead (an edge half,
+    // or a check) writes
+    const RunBounds first = run_bounds(d.row_ptr, d.n, base, lane), second = run_bounds(d.col_ptr, d.n, base, lane);
     Real x1o = Real(0), x2o = Real(0), x0o = Real(0), di = Real(0), dg = Real(1);
     if (owner) {
         x2o = d.x2[i];
@@ -373,7 +393,9 @@ __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, c
             x0o = d.x0[i];
         }
     }
-    const Real s = scatter_at<Real, Real, Wide, Pull>(d, ys, yc, base, lane, stage);
+    wait();
+    if (skip(c, gate)) return;
+    const Real s = scatter_at<Real, Real, Wide, Pull>(d, first, second, ys, yc, lane, stage);
     double acc[kNodeSums] = {0.0, 0.0, 0.0};
     if (owner) {
         Real x1v;
@@ -410,21 +432,22 @@ template <class Real, bool Reflect, bool Check, bool Wide = false, bool Pull = f
 __global__ void __launch_bounds__(kBlock)
 node_kernel(Dev<Real> d, const Real* __restrict__ ys, const Real* __restrict__ yc, int step,
             int bounds_at_1, int gate) {
-    pdl_wait();
-    pdl_launch_dependents();
-    node_kernel_tile<Real, Reflect, Check, Wide, Pull>(d, blockIdx.x, ys, yc, step, bounds_at_1, gate);
+    node_kernel_tile<Real, Reflect, Check, Wide, Pull>(d, blockIdx.x, ys, yc, step, bounds_at_1, gate, PdlWait());
 }
 
 // Dual half of one PDHG step (solver.py:269-273, projection.py:16-42) in the
 // one-coordinate form, plus the prediction of the next step's combined dual.
 // Each thread takes kEdgesPerThread edges a block-stride apart, so all their
 // loads are in flight together.
-template <class Real, bool Reflect, bool Check, bool Pull = false, int EPT = kEdgesPerThread>
-__device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, const Real* ysrc, int step, int bounds_at_1, int gate) {
+template <class Real, bool Reflect, bool Check, bool Pull = false, int EPT = kEdgesPerThread, class Wait = NoWait>
+__device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, const Real* ysrc, int step, int bounds_at_1,
+                                                 int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    if (skip(c, gate)) return;
     __shared__ double scratch[kEdgeSums * 32];
     const int base = tile * (kBlock * EPT) + threadIdx.x;
+    // the edges' constants, their dual and anchor, the control block: nothing
+    // the kernel ahead (the node half) writes
+    const bool off = skip(c, gate);
     const Real hs = Real(0.5 * kEta * c->omega);
     const double kn = Reflect ? double(c->restart_iter + step + 2) : 1.0;
     const Real lwn = Real(kn / (kn + 1.0)), rwn = Real(1.0 / (kn + 1.0));
@@ -442,6 +465,8 @@ __device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, c
             at1[t] = Pull ? e : d.colpos[e];
         }
     }
+    wait();
+    if (off) return;
     Real ri[EPT], rj[EPT];
 #pragma unroll
     for (int t = 0; t < EPT; ++t) {
@@ -497,35 +522,39 @@ __device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, c
 template <class Real, bool Reflect, bool Check, bool Pull = false>
 __global__ void __launch_bounds__(kBlock)
 edge_kernel(Dev<Real> d, const Real* ysrc, int step, int bounds_at_1, int gate) {
-    pdl_wait();
-    pdl_launch_dependents();
-    edge_kernel_tile<Real, Reflect, Check, Pull>(d, blockIdx.x, ysrc, step, bounds_at_1, gate);
+    edge_kernel_tile<Real, Reflect, Check, Pull, kEdgesPerThread>(d, blockIdx.x, ysrc, step, bounds_at_1, gate, PdlWait());
 }
 
 // The reflected step without check sums, on its own grid (tiles of kBlock *
-// plain_edges_per_thread<Real, Pull>() edges).
+// plain_edges_per_thread<Real, Pull>() edges).  The loads before the wait hold
+// more registers, so the CTAs an SM holds are pinned: FP64 4 (3 unpinned: 6.36
+// against 6.22 ms a solve at n = 4e5, m = 4e6), FP32 pull 5 (6: 27.3 against
+// 26.4 ms at n = 2e6, m = 2e7), FP32 push 8.
 template <class Real, bool Pull = false>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, sizeof(Real) == 8 ? 4 : Pull ? 5 : 8)
 edge_plain_kernel(Dev<Real> d, const Real* ysrc, int step, int bounds_at_1, int gate) {
-    pdl_wait();
-    pdl_launch_dependents();
-    edge_kernel_tile<Real, true, false, Pull, plain_edges_per_thread<Real, Pull>()>(d, blockIdx.x, ysrc, step, bounds_at_1, gate);
+    edge_kernel_tile<Real, true, false, Pull, plain_edges_per_thread<Real, Pull>()>(d, blockIdx.x, ysrc, step, bounds_at_1,
+                                                                                  gate, PdlWait());
 }
 
 // The node part of the lower bound, sum_i min(d_i - (S^T y)_i, 0), at the
 // dual (ys, yc) (solver.py:333-337), in FP64.
-template <class Real, bool Wide = false, bool Pull = false>
-__device__ __forceinline__ void lower_kernel_tile(const Dev<Real>& d, int tile, const Real* ys, const Real* yc) {
-    if (d.ctl->terminated) return;
+template <class Real, bool Wide = false, bool Pull = false, class Wait = NoWait>
+__device__ __forceinline__ void lower_kernel_tile(const Dev<Real>& d, int tile, const Real* ys, const Real* yc,
+                                                  Wait wait = Wait()) {
     __shared__ double scratch[32];
     Real* stage = warp_stage<Real, stage_runs<Wide>()>();
     const int lane = threadIdx.x & 31;
     const long long base = (long long)tile * blockDim.x + (threadIdx.x & ~31);
     const long long i = base + lane;
-    const double s = scatter_at<Real, double, Wide, Pull>(d, ys, yc, base, lane, stage);
+    const RunBounds first = run_bounds(d.row_ptr, d.n, base, lane), second = run_bounds(d.col_ptr, d.n, base, lane);
+    const Real di = i < d.n ? d.diag[i] : Real(0);
+    wait();
+    if (d.ctl->terminated) return;
+    const double s = scatter_at<Real, double, Wide, Pull>(d, first, second, ys, yc, lane, stage);
     double acc[1] = {0.0};
     if (i < d.n) {
-        const double rc = double(d.diag[i]) - s;
+        const double rc = double(di) - s;
         acc[0] = rc < 0.0 ? rc : 0.0;
     }
     block_sums<1>(acc, scratch, acc);
@@ -535,9 +564,7 @@ __device__ __forceinline__ void lower_kernel_tile(const Dev<Real>& d, int tile, 
 template <class Real, bool Wide = false, bool Pull = false>
 __global__ void __launch_bounds__(kBlock)
 lower_kernel(Dev<Real> d, const Real* __restrict__ ys, const Real* __restrict__ yc) {
-    pdl_wait();
-    pdl_launch_dependents();
-    lower_kernel_tile<Real, Wide, Pull>(d, blockIdx.x, ys, yc);
+    lower_kernel_tile<Real, Wide, Pull>(d, blockIdx.x, ys, yc, PdlWait());
 }
 
 __device__ __forceinline__ double canonical(const double* node, const double* edge, double omega) {
