@@ -171,14 +171,16 @@ bj_y(const pria::Dev<Real>* devs, const int2* __restrict__ tiles, const int* cou
 
 // Persistent clusters: cluster c takes tasks c, c + clusters, ...; every CTA
 // of a cluster takes the same task (the z half-step of one period block).
-template <class Real, int kThreads, bool Reflect, bool Check>
+// Solo: clusters of one, as plain CTAs (the same sums; a launch with the
+// cluster attribute costs microseconds more).
+template <class Real, int kThreads, bool Reflect, bool Check, bool Solo = false>
 __global__ void __launch_bounds__(kThreads)
 bj_z(const pria::Dev<Real>* devs, const int2* __restrict__ tasks, const int* count, int csize, int step,
      int gate) {
     __shared__ pria::Dev<Real> slot[2];
     const int nclusters = int(gridDim.x) / csize;
     walk_tasks(devs, tasks, *count, int(blockIdx.x) / csize, nclusters, slot, [&](const pria::Dev<Real>& sd, int2 w) {
-        pria::z_task<Real, kThreads, Reflect, Check>(sd, w.y, Reflect ? sd.zh : sd.z2s, step, gate);
+        pria::z_task<Real, kThreads, Reflect, Check, Solo>(sd, w.y, Reflect ? sd.zh : sd.z2s, step, gate);
     });
 }
 
@@ -646,6 +648,11 @@ struct Engine final : EngineBase {
         constexpr int kT = pria::z_threads<Real>();
         const int per_sm = std::max(1, int((228 * 1024) / (yz_smem[c] + 4096)));
         const int nclusters = std::max(1, (sms * std::min(per_sm, 2)) / c);
+        if (c == 1) {
+            bj_z<Real, kT, R, C, true><<<nclusters, kT, yz_smem[c], st>>>(jdevs.buf.ptr, t_yz[c].buf.ptr,
+                                                                         counts.ptr + kYZ0 + c, c, step, gate);
+            return cudaGetLastError();
+        }
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(unsigned(nclusters * c));
         cfg.blockDim = dim3(kT);
@@ -687,6 +694,9 @@ struct Engine final : EngineBase {
             RB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pria::z_slice_bytes<Real>()));
             return cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         };
+        RB_CUDA_TRY(ya(bj_z<Real, kT, true, false, true>));
+        RB_CUDA_TRY(ya(bj_z<Real, kT, true, true, true>));
+        RB_CUDA_TRY(ya(bj_z<Real, kT, false, true, true>));
         RB_CUDA_TRY(ya(bj_z<Real, kT, true, false>));
         RB_CUDA_TRY(ya(bj_z<Real, kT, true, true>));
         RB_CUDA_TRY(ya(bj_z<Real, kT, false, true>));

@@ -263,7 +263,10 @@ template <class Real, int TW, bool Reflect, bool Check>
 __device__ __forceinline__ void x_kernel_tile(const Dev<Real>& d, int tile, const Real* xsrc, const Real* ysrc, const Real* zsrc,
          int step, int gate) {
     const Control* c = d.ctl;
-    if (skip(c, gate)) return;
+    // The control block is read with the tile's data, not before it, and the
+    // decision to leave taken once the first pass has filled the tile: waiting
+    // for it first costs a round trip to L2 that nothing else fills.
+    const bool leave = skip(c, gate);
     // The tile of pre = x - tau (h + y + z) is FP64 whatever Real is: tau h
     // can exceed x by many orders of magnitude (the duals' scale is K / scale
     // per entry, the primal's is 1), and the column threshold cancels that
@@ -283,6 +286,10 @@ __device__ __forceinline__ void x_kernel_tile(const Dev<Real>& d, int tile, cons
     const int col = lane % TW, sub = lane / TW;
     const int tt = t0 + col;
     const double om = c->omega;
+    const double kn = Reflect ? double(c->restart_iter + step + 2) : 1.0;
+    // this warp's first column's last threshold, fetched with the data as well
+    double* const slot0 = d.thx + (long long)item * d.tp + (t0 + min(warp, tcols - 1));
+    const double warm0 = *slot0;
     const double tau = d.eta / om, sigma = d.eta * om;
     constexpr int kUnroll = x_unroll<Real>();
     // rows are taken kUnroll at a time per warp so that their loads are in
@@ -312,18 +319,18 @@ __device__ __forceinline__ void x_kernel_tile(const Dev<Real>& d, int tile, cons
                 pre[col * stride + sb + u * rstep] =
                     double(xv[u]) - tau * ((double(hv[u]) + double(yv[u])) + double(zv[u]));
     }
+    if (leave) return;
     __syncthreads();
+    const double lwn = kn / (kn + 1.0), rwn = 1.0 / (kn + 1.0);
     for (int cc = warp; cc < tcols; cc += nwarps) {
         double* slot = d.thx + (long long)item * d.tp + (t0 + cc);
-        const double th = michelot_smem(pre + cc * stride, t0 + cc + 1, 1.0, *slot);
+        const double th = michelot_smem(pre + cc * stride, t0 + cc + 1, 1.0, cc == warp ? warm0 : *slot);
         if (lane == 0) {
             theta[cc] = th;
             *slot = th;
         }
     }
     __syncthreads();
-    const double kn = Reflect ? double(c->restart_iter + step + 2) : 1.0;
-    const double lwn = kn / (kn + 1.0), rwn = 1.0 / (kn + 1.0);
     // Without Reflect: a vanilla step (the next point is the step itself and
     // the anchor stays), or the step that makes the point stepped from the
     // new anchor (restart; the end of the vanilla phase, whose drift sums are
@@ -386,16 +393,19 @@ x_kernel(Dev<Real> d, const Real* xsrc, const Real* __restrict__ ysrc, const Rea
 // (Michelot over the row staged in the warp's slice of shared memory,
 // warm-started from the row's last threshold), the next combined y, and at
 // checks y2 and the y parts of the check sums.  `rows` holds
-// (threads / 32) * row_cap reals, row_cap >= Tp.
-template <class Real, bool Reflect, bool Check>
+// (threads / 32) * row_cap reals, row_cap >= Tp.  A CTA of kParts times
+// kYThreads takes kParts tiles, kParts * tile and on, each by kYThreads threads
+// with sums of its own, in the order one CTA per tile adds them.
+template <class Real, bool Reflect, bool Check, int kParts = 1>
 __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, const Real* ysrc, int step, int gate,
                                               Real* rows, int row_cap) {
     const Control* c = d.ctl;
-    if (skip(c, gate)) return;
-    __shared__ double scratch[3 * 32];
+    const bool leave = skip(c, gate);   // (as in the x half-step: decided behind the row's loads)
+    constexpr int kRows = kYThreads / 32;   // rows a tile
+    __shared__ double scratch[kParts][3][kRows];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Real* v = rows + size_t(warp) * row_cap;
-    const long long g = (long long)tile * (blockDim.x >> 5) + warp;
+    const long long g = (long long)tile * (kParts * kRows) + warp;
     const double kn = Reflect ? double(c->restart_iter + step + 2) : 1.0;
     const Real lwn = Real(kn / (kn + 1.0)), rwn = Real(1.0 / (kn + 1.0));
     // Without Reflect: a vanilla step (next = the step, anchor kept) or the
@@ -409,6 +419,8 @@ __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, cons
         const int len = index_ok(blk(d.n, d.tp, s) + (long long)(i + 1) * (d.tp - s) <= d.nd, &d.ctl->status)
                             ? d.tp - s : 0;
         const long long e0 = blk(d.n, d.tp, s) + (long long)i * (d.tp - s);
+        double* slot = d.thy + (long long)s * d.n + i;
+        const double warm = *slot, target = double(d.k[i]);   // fetched with the row
         // chunks of kYChunk values per lane, loaded by predicated loads with
         // no loop around them, so each chunk is one memory round trip (an
         // unrolled loop over the row would end in a remainder loop that waits
@@ -431,9 +443,9 @@ __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, cons
                 if (q < len) v[q] = a[u] + b[u];
             }
         }
+        if (leave) return;
         __syncwarp();
-        double* slot = d.thy + (long long)s * d.n + i;
-        const double th = michelot_smem(v, len, double(d.k[i]), *slot);
+        const double th = michelot_smem(v, len, target, warm);
         if (lane == 0) *slot = th;
         for (int q0 = 0; q0 < len; q0 += 32 * kYChunk) {   // uniform over the warp
             Real y1v[kYChunk], ydv[kYChunk], dxv[kYChunk];
@@ -466,15 +478,29 @@ __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, cons
             }
         }
     }
-    if (Check) {
-        block_sums<3>(acc, scratch, acc);
-        if (threadIdx.x == 0)
-            for (int k = 0; k < 3; ++k) d.py[size_t(tile) * 3 + k] = acc[k];
+    if (leave) return;   // (the warps past the last row)
+    if (Check) {   // block_sums over each tile's threads
+        const int part = warp / kRows, w = warp % kRows;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double t = warp_sum(acc[k]);
+            if (lane == 0) scratch[part][k][w] = t;
+        }
+        __syncthreads();
+        const long long at = (long long)tile * kParts + part;
+        if (w == 0 && at * kRows < (long long)d.tp * d.n) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double t = warp_sum(lane < kRows ? scratch[part][k][lane] : 0.0);
+                if (lane == 0) d.py[size_t(at) * 3 + k] = t;
+            }
+        }
+        __syncthreads();
     }
 }
 
 template <class Real, bool Reflect, bool Check>
-__global__ void __launch_bounds__(kYThreads)
+__global__ void __launch_bounds__(kYThreads, sizeof(Real) == 4 && !Check ? 5 : 4)   // (no fewer CTAs for the early loads)
 y_kernel(Dev<Real> d, const Real* ysrc, int step, int gate) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     y_kernel_tile<Real, Reflect, Check>(d, blockIdx.x, ysrc, step, gate, reinterpret_cast<Real*>(smem_raw), d.tp);
@@ -606,7 +632,12 @@ __device__ __forceinline__ void cluster_sums(const double (&v)[K], double (*slot
 template <class Real, int kThreads, bool Reflect, bool Check, bool Solo = false>
 __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zsrc, int step, int gate) {
     const Control* c = d.ctl;
-    if (skip(c, gate)) return;   // uniform over the cluster: c is not written here
+    // Uniform over the cluster: c is not written here.  One CTA per block, a
+    // small step, decides behind its loads as the x half-step does and fetches
+    // its last threshold with them; in a cluster's longer task that bought
+    // nothing (N = 100, T = 500: 150.7 against 149.7 us for y and z).
+    const bool leave = skip(c, gate);
+    if (!Solo && leave) return;
     ZGroup<Solo> cluster;
     const int csize = Solo ? 1 : d.csize;
     const int rank = cluster.rank();
@@ -630,6 +661,7 @@ __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zs
     // v(q) = z + r of the slice's element q, in the same arithmetic either way
     auto vval = [&](int q) -> Real { return staged ? vz[q] : Real(zsrc[sbase + q] + d.r[sbase + q]); };
 
+    double warm = Solo ? d.thz[s] : 0.0;
     // phase A: z + r of the slice into shared memory, kZUnroll loads in flight
     for (int qb = threadIdx.x; staged && qb < mine; qb += kThreads * kZUnroll) {
         Real zv[kZUnroll], rv[kZUnroll];
@@ -649,7 +681,9 @@ __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zs
             if (q < mine) vz[q] = zv[u] + rv[u];
         }
     }
+    if (Solo && leave) return;
     __syncthreads();
+    if (!Solo) warm = d.thz[s];
 
     // phase B: the z threshold over the whole block, across the cluster.
     // Each CTA's (sum, count) over its slice goes to part[parity]; after one
@@ -672,7 +706,7 @@ __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zs
         C = int(t[1]);
         parity ^= 1;
     };
-    const double thz = michelot(active, d.n * len, double(d.k0), d.thz[s]);
+    const double thz = michelot(active, d.n * len, double(d.k0), warm);
     cluster.sync();   // no CTA leaves while another may still read its partials
     if (rank == 0 && threadIdx.x == 0) d.thz[s] = thz;
 
@@ -896,6 +930,27 @@ constexpr auto z_entry() {
         return z_kernel<Real, kThreads, Reflect, Check, Pair>;
 }
 
+// The y and z half-steps, independent given r, as one launch: the first Tp
+// CTAs take a period block of z each (z_task in its one-CTA form), the others
+// kParts y tiles.  Taken wherever every z block fits one CTA.  A small step is
+// launches and chains of load latencies, which then run side by side, and a
+// launch with the cluster attribute costs microseconds more than a plain one
+// even for clusters of one.  Per solve, two launches against one (FP32 / FP64):
+// N = 30, T = 75 1.80 against 1.24 / 1.78 against 1.24 ms; 40, 120 2.82 against
+// 2.14 / 2.84 against 2.06; 100, 100 4.11 against 3.12 / 4.23 against 3.43; 60,
+// 200 5.20 against 4.31 / 5.88 against 5.36 (16 waves of CTAs that hold a z
+// block's shared memory, and still faster).
+template <class Real, int kThreads, bool Reflect, bool Check>
+__global__ void __launch_bounds__(kThreads)
+yz_kernel(Dev<Real> d, const Real* ysrc, const Real* zsrc, int step, int gate) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (int(blockIdx.x) < d.tp)
+        z_task<Real, kThreads, Reflect, Check, true>(d, int(blockIdx.x), zsrc, step, gate);
+    else
+        y_kernel_tile<Real, Reflect, Check, kThreads / kYThreads>(d, int(blockIdx.x) - d.tp, ysrc, step, gate,
+                                                                  reinterpret_cast<Real*>(smem_raw), d.tp);
+}
+
 // The primal bound terms at x for period block s (solver.py:347-365):
 // sum_i K_i max_{t>=s} x_ist, K0 max_{i, t>=s} x_ist and sum h x over the
 // block, restricted to t < tlimit and s < tlimit (tlimit = t for the unpadded
@@ -1013,6 +1068,21 @@ template <class Real>
 __global__ void __launch_bounds__(kAuxThreads)
 lower_kernel(Dev<Real> d, const Real* __restrict__ y, const Real* __restrict__ z) {
     lower_kernel_tile<Real>(d, blockIdx.x, y, z);
+}
+
+// Both bounds of a check in one launch: they are independent, and short next to
+// a launch (N = 30, T = 75: 12.3 us against 10.7 + 8.7 as two; 60, 200: 25.0
+// against 14.8 + 12.8).  Taken up to kBoundsCtas CTAs, about five an SM: beyond,
+// the upper bound's long CTAs share the SMs with the other's (60, 365: 62.6
+// against 27.1 + 20.9 us; 100, 500: 124 against 51 + 41).
+constexpr int kBoundsCtas = 740;
+template <class Real>
+__global__ void __launch_bounds__(kAuxThreads)
+bounds_kernel(Dev<Real> d, const Real* __restrict__ x, const Real* __restrict__ y, const Real* __restrict__ z) {
+    if (int(blockIdx.x) < d.tp)
+        upper_kernel_tile<Real>(d, int(blockIdx.x), x, d.tp, 0);
+    else
+        lower_kernel_tile<Real>(d, int(blockIdx.x) - d.tp, y, z);
 }
 
 __device__ __forceinline__ double canonical(const double* xs, const double* yzs, double omega,
@@ -1562,7 +1632,7 @@ struct Solver final : SolverBase {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t done[2] = {nullptr, nullptr};
-    long long nlaunch = 0, block_nodes = 0;
+    long long nlaunch = 0, block_nodes = 0, step_nodes = 3, bound_nodes = 2;
     bool gated = false;   // the captured block is the conditional (gated) graph
     int runs = 0;
     // The persistent kernel (mega_block_kernel) in place of the graph: chosen
@@ -1708,7 +1778,9 @@ struct Solver final : SolverBase {
         // per row; z_task_pair) in FP64 when the pairs still fill a wave of
         // two CTAs per SM.  Measured per solve: FP64 pairs are 6-14 % faster
         // at N = 10..200, T = 300..1000; in FP32 (two z CTAs per SM) and on
-        // grids under a wave, pairs are 1-7 % slower.
+        // grids under a wave, pairs are 1-7 % slower; so are they than y and z in
+        // one launch, which blocks that fit one CTA take (yz_kernel; N = 5,
+        // T = 600 FP64 5.80 against 4.53 ms, 16, 600 11.6 against 10.6).
         auto cluster_for = [&](int row) {
             int c = 1;
             while (c < kMaxCluster && size_t((n + c - 1) / c) * row * sizeof(Real) > size_t(z_slice_bytes<Real>())) ++c;
@@ -1719,7 +1791,7 @@ struct Solver final : SolverBase {
             int dev = 0, sms = 0;
             RB_CUDA_TRY(cudaGetDevice(&dev));
             RB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            d.zpair = sizeof(Real) == 8 && (long long)(tp / 2) * csize >= 2LL * sms ? 1 : 0;
+            d.zpair = sizeof(Real) == 8 && cluster_for(tp) > 1 && (long long)(tp / 2) * csize >= 2LL * sms ? 1 : 0;
             // REFORM_PRIA_ZPAIR=0|1 overrides the choice (tests, measurements)
             const char* env = std::getenv("REFORM_PRIA_ZPAIR");
             if (env && (env[0] == '0' || env[0] == '1') && env[1] == '\0') d.zpair = env[0] - '0';
@@ -1770,7 +1842,11 @@ struct Solver final : SolverBase {
         prm.omega0 = p.omega;
         prm.vanilla_solve = p.use_halpern ? 0 : 1;
         RB_CUDA_TRY(set_attributes());
-        block_nodes = 3LL * p.op_steps + 3 + 4;   // x, y, z per step; bounds, check; restart x, y, z, check
+        choose_fused();
+        // x, y, z (or x, y and z) per step; bounds, check; a restart step, check
+        step_nodes = fused ? 2 : 3;
+        bound_nodes = tp + nblo <= kBoundsCtas ? 1 : 2;
+        block_nodes = step_nodes * p.op_steps + bound_nodes + 1 + step_nodes + 1;
         RB_CUDA_TRY(init_mega());
         return cudaGetLastError();
     }
@@ -1802,8 +1878,12 @@ struct Solver final : SolverBase {
         // REFORM_PRIA_MEGA=0|1 sets the initial mode (tests, measurements);
         // REFORM_PRIA_MEGA_PHANTOM=k makes every barrier wait for k CTAs that
         // are never launched, so each wait runs out (the fault-injection test)
+        // Unless asked for, a solver takes the graph: since y and z share a
+        // launch it is the faster form at every size (per solve, FP64: N = 3,
+        // T = 10 0.66 against 1.16 ms; 10, 25 0.91 against 1.51; 20, 40 1.00
+        // against 1.76).
         const char* env = std::getenv("REFORM_PRIA_MEGA");
-        int mode = -1;
+        int mode = 0;
         if (env && (env[0] == '0' || env[0] == '1') && env[1] == '\0') mode = env[0] - '0';
         const char* ph = std::getenv("REFORM_PRIA_MEGA_PHANTOM");
         if (ph) {
@@ -1854,6 +1934,8 @@ struct Solver final : SolverBase {
     static cudaError_t yz_attr() {
         RB_CUDA_TRY(cudaFuncSetAttribute(y_kernel<Real, R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(y_smem_limit())));
+        RB_CUDA_TRY(cudaFuncSetAttribute(yz_kernel<Real, z_threads<Real>(), R, C>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, z_slice_bytes<Real>()));
         for (auto fn : {z_entry<Real, z_threads<Real>(), R, C, false>(), z_entry<Real, z_threads<Real>(), R, C, true>()}) {
             RB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, z_slice_bytes<Real>()));
             RB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -1892,11 +1974,29 @@ struct Solver final : SolverBase {
         return cudaGetLastError();
     }
 
+    // y and z in one launch (yz_kernel): its CTAs and shared memory
+    static constexpr int kYParts = z_threads<Real>() / kYThreads;
+    bool fused = false;
+    int fused_grid() const { return tp + (nby + kYParts - 1) / kYParts; }
+    size_t fused_smem() const {
+        return std::max(yz_smem, size_t(z_threads<Real>() / 32) * tp * sizeof(Real));
+    }
+    void choose_fused() {
+        const char* env = std::getenv("REFORM_PRIA_FUSE");   // 0: never (tests, measurements)
+        fused = d.csize == 1 && !d.zpair && d.zstaged && fused_smem() <= size_t(z_slice_bytes<Real>()) &&
+                !(env && !std::strcmp(env, "0"));
+    }
+
     template <bool R, bool C>
     // the y half-step (one warp per row) and then the z half-step (a cluster
     // per z task: a period block, or a pair of them); two launches
     cudaError_t launch_yz(const Real* ys, const Real* zs, int step, int gate, cudaStream_t on = nullptr) {
         cudaStream_t st = on ? on : stream;
+        if (fused) {
+            yz_kernel<Real, z_threads<Real>(), R, C><<<fused_grid(), z_threads<Real>(), fused_smem(), st>>>(d, ys, zs, step,
+                                                                                                          gate);
+            return cudaGetLastError();
+        }
         y_kernel<Real, R, C><<<nby, kYThreads, size_t(kYThreads / 32) * tp * sizeof(Real), st>>>(d, ys, step, gate);
         RB_CUDA_TRY(cudaGetLastError());
         cudaLaunchConfig_t cfg = {};
@@ -1913,6 +2013,16 @@ struct Solver final : SolverBase {
         cfg.numAttrs = 1;
         if (d.zpair) return cudaLaunchKernelEx(&cfg, z_entry<Real, z_threads<Real>(), R, C, true>(), d, zs, step, gate);
         return cudaLaunchKernelEx(&cfg, z_entry<Real, z_threads<Real>(), R, C, false>(), d, zs, step, gate);
+    }
+
+    cudaError_t launch_bounds_at(const Real* x, const Real* y, const Real* z) {
+        if (bound_nodes == 1) {
+            bounds_kernel<Real><<<tp + nblo, kAuxThreads, 0, stream>>>(d, x, y, z);
+        } else {
+            upper_kernel<Real><<<tp, kAuxThreads, 0, stream>>>(d, x, tp, 0);
+            lower_kernel<Real><<<nblo, kAuxThreads, 0, stream>>>(d, y, z);
+        }
+        return cudaGetLastError();
     }
 
     cudaError_t launch_check(int mode) {
@@ -1963,8 +2073,7 @@ struct Solver final : SolverBase {
                 RB_PTIMED(3, (launch_yz<true, true>(d.yh, d.zh, s, 0)));
             }
         }
-        RB_PTIMED(4, (upper_kernel<Real><<<tp, kAuxThreads, 0, stream>>>(d, d.x2s, tp, 0), cudaGetLastError()));
-        RB_PTIMED(5, (lower_kernel<Real><<<nblo, kAuxThreads, 0, stream>>>(d, d.y2s, d.z2s), cudaGetLastError()));
+        RB_PTIMED(4, launch_bounds_at(d.x2s, d.y2s, d.z2s));   // (both bounds: kind 5 is not used)
         RB_PTIMED(6, launch_check(1));
         RB_PTIMED(7, (launch_x<false, true>(d.x2s, d.y2s, d.z2s, 0, 1)));
         RB_PTIMED(7, (launch_yz<false, true>(d.y2s, d.z2s, 0, 1)));
@@ -2100,13 +2209,12 @@ struct Solver final : SolverBase {
         // x1 = raw_step(x0): one vanilla step from the start point, with the
         // sums for the error, and the bounds at the start point itself.
         RB_CUDA_TRY(cudaGetLastError());
-        upper_kernel<Real><<<tp, kAuxThreads, 0, stream>>>(d, d.x0, tp, 0);
-        lower_kernel<Real><<<nblo, kAuxThreads, 0, stream>>>(d, d.y0, d.z0);
+        RB_CUDA_TRY(launch_bounds_at(d.x0, d.y0, d.z0));
         RB_CUDA_TRY((launch_x<false, true>(d.x0, d.y0, d.z0, 0, 0)));
         RB_CUDA_TRY((launch_yz<false, true>(d.y0, d.z0, 0, 0)));
         RB_CUDA_TRY(launch_check(0));
         RB_CUDA_TRY(cudaMemcpyAsync(mirror, d.ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream));
-        nlaunch += 6;
+        nlaunch += bound_nodes + 1 + step_nodes;
         return cudaStreamSynchronize(stream);
     }
 
@@ -2122,10 +2230,9 @@ struct Solver final : SolverBase {
             RB_CUDA_TRY((launch_x<false, false>(d.xh, d.yh, d.zh, 0, kGateVanilla)));
             RB_CUDA_TRY((launch_yz<false, false>(d.yh, d.zh, 0, kGateVanilla)));
         }
-        upper_kernel<Real><<<tp, kAuxThreads, 0, stream>>>(d, d.xh, tp, 0);
-        lower_kernel<Real><<<nblo, kAuxThreads, 0, stream>>>(d, d.yh, d.zh);
+        RB_CUDA_TRY(launch_bounds_at(d.xh, d.yh, d.zh));
         RB_CUDA_TRY(launch_check(3));
-        nlaunch += 3LL * p.op_steps + 3;
+        nlaunch += step_nodes * p.op_steps + bound_nodes + 1;
         return cudaMemcpyAsync(mirror, d.ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream);
     }
 
@@ -2160,7 +2267,7 @@ struct Solver final : SolverBase {
         RB_CUDA_TRY((launch_x<false, true>(d.xh, d.yh, d.zh, 0, kGateDrift)));
         RB_CUDA_TRY((launch_yz<false, true>(d.yh, d.zh, 0, kGateDrift)));
         RB_CUDA_TRY(launch_check(4));
-        nlaunch += 4;
+        nlaunch += step_nodes + 1;
         RB_CUDA_TRY(cudaMemcpyAsync(mirror, d.ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream));
         return cudaStreamSynchronize(stream);
     }

@@ -18,6 +18,8 @@ at the same tolerance.
 import json
 from pathlib import Path
 
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -454,6 +456,36 @@ def test_persistent_kernel_vanilla_and_warm_phase(native, mode):
     _, (g,), _ = _mega_solve(inst, p, "fp64", 0)
     assert on
     _same(m, g)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,t,extra", [(1, 1, {}), (1, 2, {}), (3, 17, {}), (7, 33, {"warm_steps": 2}), (9, 64, {}),
+                                       (16, 7, {"use_halpern": 0, "max_iter": 64}), (61, 199, {}), (2, 600, {})])
+def test_y_and_z_in_one_launch_equal_two(native, monkeypatch, precision, n, t, extra):
+    """The y and z half-steps (and the two bounds) in one launch, the solver's
+    choice where a z block fits one CTA, against a launch each: the same
+    arithmetic and sums, so the same solve bit for bit.  One row, fewer rows
+    than a tile, a last tile that is not full (FP32 takes two a CTA), odd
+    horizons, both sides of the size up to which the bounds share a launch, the
+    plain and the warm phase, zero costs, largest block near a CTA's share."""
+    from reformulation_b200 import pria
+    inst = jrp_demand(40 + n, n, t)
+    if n == 9:
+        k = inst.order_costs.copy()
+        k[4] = 0.0
+        inst = dataclasses.replace(inst, order_costs=k, joint_order_cost=0.0)
+    opts = {"max_iter": 400, "tolerance": 1e-6} | extra
+    p = pria.Library().parameters(**opts)
+    out = []
+    for fuse in ("1", "0"):
+        monkeypatch.setenv("REFORM_PRIA_FUSE", fuse)
+        with pria.DeviceSolver(inst, p, precision) as dev:
+            for _ in range(2):
+                assert dev.run() == 0
+            out.append((dev.result(want_solution=True), dev.launches()))
+    (a, la), (b, lb) = out
+    _same(a, b)
+    assert la < lb or a.iterations == 0
 
 
 def test_persistent_kernel_choice(native):
