@@ -5,6 +5,7 @@
 // on the launch shape only, so a solve is bitwise reproducible run to run).
 #pragma once
 
+#include <type_traits>
 #include <utility>
 
 #include <cuda_runtime.h>
@@ -106,22 +107,45 @@ __device__ __forceinline__ void reduce_rows(const double* rows, int count, doubl
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 
-// Launch `kernel` on `stream` with the programmatic stream-serialization
-// attribute (the kernel must call pdl_wait() before it touches memory the
-// previous kernel writes).
+// What a kernel of a programmatic chain does between what it may read at once
+// and what the kernel ahead of it writes: wait for that kernel, then let the
+// next one start.  A kernel that has started found every kernel before its
+// predecessor complete (the predecessor waited for them before it let this one
+// start), so before the wait it may read the instance's constants and whatever
+// its predecessor does not write; the latency of those loads then runs beside
+// the predecessor's last CTAs.  NoWait: everything is there (persistent kernels,
+// the batched engine).
+struct NoWait {
+    __device__ __forceinline__ void operator()() const {}
+};
+struct PdlWait {
+    __device__ __forceinline__ void operator()() const {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
+};
+
+// Launch `kernel` on `stream` with `smem` bytes of dynamic shared memory and, if
+// `pdl`, with the programmatic stream-serialization attribute (the kernel must
+// call pdl_wait() before it touches memory the previous kernel writes).
 template <class... KArgs, class... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_ex(void (*kernel)(KArgs...), int grid, int block, size_t smem, bool pdl, cudaStream_t stream,
+                             Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(grid));
     cfg.blockDim = dim3(unsigned(block));
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <class... KArgs, class... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t stream, Args&&... args) {
+    return launch_ex(kernel, grid, block, 0, true, stream, std::forward<Args>(args)...);
 }
 
 // Start bringing the line of `p` into L2 (no register, no wait): for data a

@@ -156,27 +156,6 @@ constexpr int kPull = RB200_PRAQ_PULL;
 template <class Real>
 constexpr int stage_len() { return RB200_PRAQ_STAGE_BYTES / int(sizeof(Real)); }
 
-// What a kernel of a programmatic chain does between what it may read at once
-// and what the kernel ahead of it writes: wait for that kernel, then let the
-// next one start.  A kernel that has started found every kernel before its
-// predecessor complete (the predecessor waited for them before it let this one
-// start), so before the wait it may read the instance's constants and whatever
-// its predecessor does not write; the latency of those loads then runs beside
-// the predecessor's last CTAs.  (Waiting first and then reading everything:
-// n = 3,000, m = 24,000 0.56 against 0.51 ms a solve in FP32, 0.74 against 0.65
-// in FP64; 50,000, 200,000 FP64 1.16 against 1.00; 1e5, 1e6 1.41 against 1.35
-// and 1.71 against 1.64; 2e6, 2e7 26.6 against 26.4.)  NoWait: everything is
-// there (persistent kernels, the batched engine).
-struct NoWait {
-    __device__ __forceinline__ void operator()() const {}
-};
-struct PdlWait {
-    __device__ __forceinline__ void operator()() const {
-        pdl_wait();
-        pdl_launch_dependents();
-    }
-};
-
 // The runs of a warp's 32 consecutive nodes base + lane: the warp's whole
 // range [lo, hi) and this lane's own [a, b) (empty past the last node).
 struct RunBounds {
@@ -366,6 +345,11 @@ __device__ __forceinline__ Acc scatter_at(const Dev<Real>& d, const RunBounds& f
     }
 }
 
+// (Kernels that waited for their predecessor first and then read everything:
+// n = 3,000, m = 24,000 0.56 against 0.51 ms a solve in FP32, 0.74 against 0.65
+// in FP64; 50,000, 200,000 FP64 1.16 against 1.00; 1e5, 1e6 1.41 against 1.35
+// and 1.71 against 1.64; 2e6, 2e7 26.6 against 26.4.)
+//
 // Primal half of one PDHG step, with the Halpern combination of x folded in
 // (solver.py:259-267 and 276-292).  Reflect: x1 = lw (2 x2 - x1) + rw x0 with
 // k = restart_iter + step + 1; vanilla: x1 = x2 and the anchor becomes x1.

@@ -259,9 +259,9 @@ __device__ double michelot_smem(const Real* v, int len, double target, double wa
 // the next combined x.  Reflect: the point stepped from is xsrc (= xh);
 // vanilla: xsrc is the point itself and becomes the anchor.  Check: x2 and
 // x1 - x2 are kept and the x sums go to px.
-template <class Real, int TW, bool Reflect, bool Check>
+template <class Real, int TW, bool Reflect, bool Check, class Wait = NoWait>
 __device__ __forceinline__ void x_kernel_tile(const Dev<Real>& d, int tile, const Real* xsrc, const Real* ysrc, const Real* zsrc,
-         int step, int gate) {
+         int step, int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
     // The control block is read with the tile's data, not before it, and the
     // decision to leave taken once the first pass has filled the tile: waiting
@@ -295,6 +295,8 @@ __device__ __forceinline__ void x_kernel_tile(const Dev<Real>& d, int tile, cons
     // rows are taken kUnroll at a time per warp so that their loads are in
     // flight together
     const int rstep = nwarps * kRpw;
+    constexpr bool kChain = !std::is_same_v<Wait, NoWait>;
+    bool waited = !kChain;   // before the first read of y or z, which the kernel ahead writes
     for (int sb = warp * kRpw + sub; sb < rows; sb += rstep * kUnroll) {
         long long ev[kUnroll];
         Real xv[kUnroll], hv[kUnroll], yv[kUnroll], zv[kUnroll];
@@ -307,10 +309,23 @@ __device__ __forceinline__ void x_kernel_tile(const Dev<Real>& d, int tile, cons
                 ev[u] = blk(d.n, d.tp, s) + (long long)item * (d.tp - s) + (tt - s);
                 xv[u] = xsrc[ev[u]];
                 hv[u] = d.h[ev[u]];
-                yv[u] = ysrc[ev[u]];
-                zv[u] = zsrc[ev[u]];
+                if constexpr (!kChain) {
+                    yv[u] = ysrc[ev[u]];
+                    zv[u] = zsrc[ev[u]];
+                }
                 // the anchor the second pass reads, on chip by then
                 if ((Reflect || (gate & kGateDrift)) && ((col & 7) == 0 || tt == s)) prefetch_l2(d.x0 + ev[u]);
+            }
+        }
+        if constexpr (kChain) {
+            if (!waited) wait();
+            waited = true;
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                if (ev[u] >= 0) {
+                    yv[u] = ysrc[ev[u]];
+                    zv[u] = zsrc[ev[u]];
+                }
             }
         }
 #pragma unroll
@@ -319,6 +334,7 @@ __device__ __forceinline__ void x_kernel_tile(const Dev<Real>& d, int tile, cons
                 pre[col * stride + sb + u * rstep] =
                     double(xv[u]) - tau * ((double(hv[u]) + double(yv[u])) + double(zv[u]));
     }
+    if (!waited) wait();
     if (leave) return;
     __syncthreads();
     const double lwn = kn / (kn + 1.0), rwn = 1.0 / (kn + 1.0);
@@ -387,6 +403,13 @@ x_kernel(Dev<Real> d, const Real* xsrc, const Real* __restrict__ ysrc, const Rea
     x_kernel_tile<Real, TW, Reflect, Check>(d, blockIdx.x, xsrc, ysrc, zsrc, step, gate);
 }
 
+// The same in a programmatic chain with yz_kernel (small steps).
+template <class Real, int TW, bool Reflect, bool Check>
+__global__ void __launch_bounds__(kXThreads)
+x_chain_kernel(Dev<Real> d, const Real* xsrc, const Real* ysrc, const Real* zsrc, int step, int gate) {
+    x_kernel_tile<Real, TW, Reflect, Check>(d, blockIdx.x, xsrc, ysrc, zsrc, step, gate, PdlWait());
+}
+
 // y half-step (solver.py:421-422) for one tile of rows: warp w takes row
 // g = tile * (rows per tile) + w of the period-major order (block s, item i),
 // a contiguous run of Tp - s values.  y' = P_Y(y + r) onto the K_i simplex
@@ -396,9 +419,9 @@ x_kernel(Dev<Real> d, const Real* xsrc, const Real* __restrict__ ysrc, const Rea
 // (threads / 32) * row_cap reals, row_cap >= Tp.  A CTA of kParts times
 // kYThreads takes kParts tiles, kParts * tile and on, each by kYThreads threads
 // with sums of its own, in the order one CTA per tile adds them.
-template <class Real, bool Reflect, bool Check, int kParts = 1>
+template <class Real, bool Reflect, bool Check, int kParts = 1, class Wait = NoWait>
 __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, const Real* ysrc, int step, int gate,
-                                              Real* rows, int row_cap) {
+                                              Real* rows, int row_cap, Wait wait = Wait()) {
     const Control* c = d.ctl;
     const bool leave = skip(c, gate);   // (as in the x half-step: decided behind the row's loads)
     constexpr int kRows = kYThreads / 32;   // rows a tile
@@ -425,6 +448,8 @@ __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, cons
         // no loop around them, so each chunk is one memory round trip (an
         // unrolled loop over the row would end in a remainder loop that waits
         // for every load in turn)
+        constexpr bool kChain = !std::is_same_v<Wait, NoWait>;
+        bool waited = !kChain;   // before the first read of r, which the kernel ahead writes
         for (int q0 = 0; q0 < len; q0 += 32 * kYChunk) {   // uniform over the warp
             Real a[kYChunk], b[kYChunk];
 #pragma unroll
@@ -432,8 +457,17 @@ __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, cons
                 const int q = q0 + lane + 32 * u;
                 if (q < len) {
                     a[u] = ysrc[e0 + q];
-                    b[u] = d.r[e0 + q];
+                    if constexpr (!kChain) b[u] = d.r[e0 + q];
                     if (drift && (q & 7) == 0) prefetch_l2(d.y0 + e0 + q);   // one per 32-byte sector
+                }
+            }
+            if (!waited) wait();
+            waited = true;
+#pragma unroll
+            for (int u = 0; u < kYChunk; ++u) {
+                const int q = q0 + lane + 32 * u;
+                if (q < len) {
+                    if constexpr (kChain) b[u] = d.r[e0 + q];
                     if (Check && (q & 7) == 0) prefetch_l2(d.dxs + e0 + q);
                 }
             }
@@ -443,6 +477,7 @@ __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, cons
                 if (q < len) v[q] = a[u] + b[u];
             }
         }
+        if (!waited) wait();
         if (leave) return;
         __syncwarp();
         const double th = michelot_smem(v, len, target, warm);
@@ -478,6 +513,8 @@ __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, cons
             }
         }
     }
+    else
+        wait();
     if (leave) return;   // (the warps past the last row)
     if (Check) {   // block_sums over each tile's threads
         const int part = warp / kRows, w = warp % kRows;
@@ -629,8 +666,8 @@ __device__ __forceinline__ void cluster_sums(const double (&v)[K], double (*slot
 // shared memory, then the slice's z is written.  Solo: the whole block in
 // this CTA (csize 1), CTA barriers in place of cluster barriers, the same
 // sums in the same order.
-template <class Real, int kThreads, bool Reflect, bool Check, bool Solo = false>
-__device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zsrc, int step, int gate) {
+template <class Real, int kThreads, bool Reflect, bool Check, bool Solo = false, class Wait = NoWait>
+__device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zsrc, int step, int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
     // Uniform over the cluster: c is not written here.  One CTA per block, a
     // small step, decides behind its loads as the x half-step does and fetches
@@ -663,6 +700,8 @@ __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zs
 
     double warm = Solo ? d.thz[s] : 0.0;
     // phase A: z + r of the slice into shared memory, kZUnroll loads in flight
+    constexpr bool kChain = !std::is_same_v<Wait, NoWait>;
+    bool waited = !kChain;   // before the first read of r, which the kernel ahead writes
     for (int qb = threadIdx.x; staged && qb < mine; qb += kThreads * kZUnroll) {
         Real zv[kZUnroll], rv[kZUnroll];
 #pragma unroll
@@ -670,8 +709,17 @@ __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zs
             const int q = qb + u * kThreads;
             if (q < mine) {
                 zv[u] = zsrc[sbase + q];
-                rv[u] = d.r[sbase + q];
+                if constexpr (!kChain) rv[u] = d.r[sbase + q];
                 if (drift && (q & 7) == 0) prefetch_l2(d.z0 + sbase + q);
+            }
+        }
+        if (!waited) wait();
+        waited = true;
+#pragma unroll
+        for (int u = 0; u < kZUnroll; ++u) {
+            const int q = qb + u * kThreads;
+            if (q < mine) {
+                if constexpr (kChain) rv[u] = d.r[sbase + q];
                 if (Check && (q & 7) == 0) prefetch_l2(d.dxs + sbase + q);
             }
         }
@@ -681,6 +729,7 @@ __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zs
             if (q < mine) vz[q] = zv[u] + rv[u];
         }
     }
+    if (!waited) wait();
     if (Solo && leave) return;
     __syncthreads();
     if (!Solo) warm = d.thz[s];
@@ -940,15 +989,15 @@ constexpr auto z_entry() {
 // 2.14 / 2.84 against 2.06; 100, 100 4.11 against 3.12 / 4.23 against 3.43; 60,
 // 200 5.20 against 4.31 / 5.88 against 5.36 (16 waves of CTAs that hold a z
 // block's shared memory, and still faster).
-template <class Real, int kThreads, bool Reflect, bool Check>
+template <class Real, int kThreads, bool Reflect, bool Check, class Wait>
 __global__ void __launch_bounds__(kThreads)
 yz_kernel(Dev<Real> d, const Real* ysrc, const Real* zsrc, int step, int gate) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (int(blockIdx.x) < d.tp)
-        z_task<Real, kThreads, Reflect, Check, true>(d, int(blockIdx.x), zsrc, step, gate);
+        z_task<Real, kThreads, Reflect, Check, true>(d, int(blockIdx.x), zsrc, step, gate, Wait());
     else
         y_kernel_tile<Real, Reflect, Check, kThreads / kYThreads>(d, int(blockIdx.x) - d.tp, ysrc, step, gate,
-                                                                  reinterpret_cast<Real*>(smem_raw), d.tp);
+                                                                  reinterpret_cast<Real*>(smem_raw), d.tp, Wait());
 }
 
 // The primal bound terms at x for period block s (solver.py:347-365):
@@ -1927,6 +1976,8 @@ struct Solver final : SolverBase {
     // lower the limit under an earlier, larger one.
     template <int TW, bool R, bool C>
     static cudaError_t x_attr() {
+        RB_CUDA_TRY(cudaFuncSetAttribute(x_chain_kernel<Real, TW, R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(x_smem_limit())));
         return cudaFuncSetAttribute(x_kernel<Real, TW, R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     int(x_smem_limit()));
     }
@@ -1934,8 +1985,8 @@ struct Solver final : SolverBase {
     static cudaError_t yz_attr() {
         RB_CUDA_TRY(cudaFuncSetAttribute(y_kernel<Real, R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(y_smem_limit())));
-        RB_CUDA_TRY(cudaFuncSetAttribute(yz_kernel<Real, z_threads<Real>(), R, C>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, z_slice_bytes<Real>()));
+        for (auto fn : {yz_kernel<Real, z_threads<Real>(), R, C, NoWait>, yz_kernel<Real, z_threads<Real>(), R, C, PdlWait>})
+            RB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, z_slice_bytes<Real>()));
         for (auto fn : {z_entry<Real, z_threads<Real>(), R, C, false>(), z_entry<Real, z_threads<Real>(), R, C, true>()}) {
             RB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, z_slice_bytes<Real>()));
             RB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -1970,6 +2021,9 @@ struct Solver final : SolverBase {
     template <bool R, bool C>
     cudaError_t launch_x(const Real* xs, const Real* ys, const Real* zs, int step, int gate,
                          cudaStream_t on = nullptr) {
+        if (chained && !on)   // (a step's first x follows a copy or the check: a plain launch)
+            return launch_ex(x_chain_kernel<Real, kXTile, R, C>, n * d.ntc, kXThreads, x_smem, R && step > 0, stream, d, xs,
+                             ys, zs, step, gate);
         x_kernel<Real, kXTile, R, C><<<n * d.ntc, kXThreads, x_smem, on ? on : stream>>>(d, xs, ys, zs, step, gate);
         return cudaGetLastError();
     }
@@ -1977,6 +2031,15 @@ struct Solver final : SolverBase {
     // y and z in one launch (yz_kernel): its CTAs and shared memory
     static constexpr int kYParts = z_threads<Real>() / kYThreads;
     bool fused = false;
+    // x and yz as a programmatic chain, each reading what the other does not
+    // write before it waits for it: pays while a step is short.  Per solve,
+    // plain against chained (FP32 / FP64): N = 3, T = 10 0.68 against 0.62 /
+    // 0.65 against 0.57 ms; 10, 25 0.94 against 0.84 / 0.92 against 0.79; 40,
+    // 120 2.11 against 2.00 / 2.01 against 2.03; 100, 100 (505,000 entries) 3.12
+    // against 3.13 / 3.43 against 3.33; 5, 600 (900,000) 4.90 against 5.30 /
+    // 4.53 against 5.22.
+    static constexpr long long kChainEntries = 524288;
+    bool chained = false;
     int fused_grid() const { return tp + (nby + kYParts - 1) / kYParts; }
     size_t fused_smem() const {
         return std::max(yz_smem, size_t(z_threads<Real>() / 32) * tp * sizeof(Real));
@@ -1985,6 +2048,7 @@ struct Solver final : SolverBase {
         const char* env = std::getenv("REFORM_PRIA_FUSE");   // 0: never (tests, measurements)
         fused = d.csize == 1 && !d.zpair && d.zstaged && fused_smem() <= size_t(z_slice_bytes<Real>()) &&
                 !(env && !std::strcmp(env, "0"));
+        chained = fused && nd <= kChainEntries;
     }
 
     template <bool R, bool C>
@@ -1993,9 +2057,9 @@ struct Solver final : SolverBase {
     cudaError_t launch_yz(const Real* ys, const Real* zs, int step, int gate, cudaStream_t on = nullptr) {
         cudaStream_t st = on ? on : stream;
         if (fused) {
-            yz_kernel<Real, z_threads<Real>(), R, C><<<fused_grid(), z_threads<Real>(), fused_smem(), st>>>(d, ys, zs, step,
-                                                                                                          gate);
-            return cudaGetLastError();
+            const bool chain = chained && !on;
+            auto fn = chain ? yz_kernel<Real, z_threads<Real>(), R, C, PdlWait> : yz_kernel<Real, z_threads<Real>(), R, C, NoWait>;
+            return launch_ex(fn, fused_grid(), z_threads<Real>(), fused_smem(), chain, st, d, ys, zs, step, gate);
         }
         y_kernel<Real, R, C><<<nby, kYThreads, size_t(kYThreads / 32) * tp * sizeof(Real), st>>>(d, ys, step, gate);
         RB_CUDA_TRY(cudaGetLastError());
