@@ -2402,9 +2402,15 @@ struct Solver final : SolverBase {
             if (st) return st;
         }
         // Keep one block in flight ahead of the one being inspected; blocks
-        // launched after termination see the flag and return at once.
+        // launched after termination see the flag and return at once.  A first
+        // run of the pull layout, whose blocks take milliseconds, waits for each
+        // check instead: its kernels read what they may before they see the
+        // flag, and the block too many costs 1.2 ms at n = 2e6, m = 2e7, five
+        // waits a tenth of that.  (A replayed block behind the end runs its gate
+        // alone.)
+        const int depth = pull && !exec && !mega ? 1 : 2;
         if (!mirror->terminated) {
-            for (int k = 0; k < 2; ++k) {
+            for (int k = 0; k < depth; ++k) {
                 if (launch_block() != cudaSuccess) return PRAQ_ERROR_CUDA;
                 if (cudaEventRecord(done[k], stream) != cudaSuccess) return PRAQ_ERROR_CUDA;
                 nlaunch += block_launches();
@@ -2424,7 +2430,7 @@ struct Solver final : SolverBase {
                 if (launch_block() != cudaSuccess) return PRAQ_ERROR_CUDA;
                 if (cudaEventRecord(done[k], stream) != cudaSuccess) return PRAQ_ERROR_CUDA;
                 nlaunch += block_launches();
-                k ^= 1;
+                k = (k + 1) % depth;
             }
         }
         if (cudaMemcpyAsync(mirror, d.ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||

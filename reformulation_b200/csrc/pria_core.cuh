@@ -263,10 +263,15 @@ template <class Real, int TW, bool Reflect, bool Check, class Wait = NoWait>
 __device__ __forceinline__ void x_kernel_tile(const Dev<Real>& d, int tile, const Real* xsrc, const Real* ysrc, const Real* zsrc,
          int step, int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    // The control block is read with the tile's data, not before it, and the
-    // decision to leave taken once the first pass has filled the tile: waiting
-    // for it first costs a round trip to L2 that nothing else fills.
+    // In a chain of short steps the control block is read with the tile's data,
+    // not before it, and the decision to leave taken once the first pass has
+    // filled the tile: waiting for it first costs a round trip to L2 that
+    // nothing else fills.  A long step decides first: a first run's last block,
+    // queued behind the one that ended the solve, would else read it all again
+    // (N = 100, T = 500: 34.5 against 33.2 ms for a first run).
+    constexpr bool kChain = !std::is_same_v<Wait, NoWait>;
     const bool leave = skip(c, gate);
+    if (!kChain && leave) return;
     // The tile of pre = x - tau (h + y + z) is FP64 whatever Real is: tau h
     // can exceed x by many orders of magnitude (the duals' scale is K / scale
     // per entry, the primal's is 1), and the column threshold cancels that
@@ -295,7 +300,6 @@ __device__ __forceinline__ void x_kernel_tile(const Dev<Real>& d, int tile, cons
     // rows are taken kUnroll at a time per warp so that their loads are in
     // flight together
     const int rstep = nwarps * kRpw;
-    constexpr bool kChain = !std::is_same_v<Wait, NoWait>;
     bool waited = !kChain;   // before the first read of y or z, which the kernel ahead writes
     for (int sb = warp * kRpw + sub; sb < rows; sb += rstep * kUnroll) {
         long long ev[kUnroll];
@@ -423,7 +427,9 @@ template <class Real, bool Reflect, bool Check, int kParts = 1, class Wait = NoW
 __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, const Real* ysrc, int step, int gate,
                                               Real* rows, int row_cap, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    const bool leave = skip(c, gate);   // (as in the x half-step: decided behind the row's loads)
+    constexpr bool kChain = !std::is_same_v<Wait, NoWait>;
+    const bool leave = skip(c, gate);   // (as in the x half-step)
+    if (!kChain && leave) return;
     constexpr int kRows = kYThreads / 32;   // rows a tile
     __shared__ double scratch[kParts][3][kRows];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -448,7 +454,6 @@ __device__ __forceinline__ void y_kernel_tile(const Dev<Real>& d, int tile, cons
         // no loop around them, so each chunk is one memory round trip (an
         // unrolled loop over the row would end in a remainder loop that waits
         // for every load in turn)
-        constexpr bool kChain = !std::is_same_v<Wait, NoWait>;
         bool waited = !kChain;   // before the first read of r, which the kernel ahead writes
         for (int q0 = 0; q0 < len; q0 += 32 * kYChunk) {   // uniform over the warp
             Real a[kYChunk], b[kYChunk];
@@ -669,12 +674,9 @@ __device__ __forceinline__ void cluster_sums(const double (&v)[K], double (*slot
 template <class Real, int kThreads, bool Reflect, bool Check, bool Solo = false, class Wait = NoWait>
 __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zsrc, int step, int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    // Uniform over the cluster: c is not written here.  One CTA per block, a
-    // small step, decides behind its loads as the x half-step does and fetches
-    // its last threshold with them; in a cluster's longer task that bought
-    // nothing (N = 100, T = 500: 150.7 against 149.7 us for y and z).
-    const bool leave = skip(c, gate);
-    if (!Solo && leave) return;
+    constexpr bool kChain = !std::is_same_v<Wait, NoWait>;
+    const bool leave = skip(c, gate);   // (as in the x half-step) uniform over the cluster: c is not written here
+    if (!kChain && leave) return;
     ZGroup<Solo> cluster;
     const int csize = Solo ? 1 : d.csize;
     const int rank = cluster.rank();
@@ -698,9 +700,8 @@ __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zs
     // v(q) = z + r of the slice's element q, in the same arithmetic either way
     auto vval = [&](int q) -> Real { return staged ? vz[q] : Real(zsrc[sbase + q] + d.r[sbase + q]); };
 
-    double warm = Solo ? d.thz[s] : 0.0;
+    double warm = kChain ? d.thz[s] : 0.0;   // fetched with the slice
     // phase A: z + r of the slice into shared memory, kZUnroll loads in flight
-    constexpr bool kChain = !std::is_same_v<Wait, NoWait>;
     bool waited = !kChain;   // before the first read of r, which the kernel ahead writes
     for (int qb = threadIdx.x; staged && qb < mine; qb += kThreads * kZUnroll) {
         Real zv[kZUnroll], rv[kZUnroll];
@@ -730,9 +731,9 @@ __device__ __forceinline__ void z_task(const Dev<Real>& d, int s, const Real* zs
         }
     }
     if (!waited) wait();
-    if (Solo && leave) return;
+    if (leave) return;
     __syncthreads();
-    if (!Solo) warm = d.thz[s];
+    if (!kChain) warm = d.thz[s];
 
     // phase B: the z threshold over the whole block, across the cluster.
     // Each CTA's (sum, count) over its slice goes to part[parity]; after one
