@@ -461,7 +461,7 @@ def sub_pria(timer, steps, skip_cpu):
 def sub_pria_small(timer, steps, skip_cpu):
     """Small JRPs, latency-bound: N=10, T=25 and N=30, T=75 (seeds 5, 6), to
     1e-4.  Device-resident solves from the cold start with the solver's
-    automatic choice beside the per-kernel graph and the persistent kernel
+    own choice beside the per-kernel graph and the persistent kernel
     (one cooperative launch per check block) forced on, mixed and FP64;
     solves through pria_solve with host buffers; the CPU restatement on one
     thread."""
@@ -476,9 +476,9 @@ def sub_pria_small(timer, steps, skip_cpu):
         p = lib.parameters(1_000_000, TOL)
         rec = {"entries": inst.entries}
         for prec in ("mixed", "fp64"):
-            for mode, name in ((-1, "auto"), (0, "graph"), (1, "persistent")):
+            for mode, name in ((None, "auto"), (0, "graph"), (1, "persistent")):
                 with pria.DeviceSolver(inst, p, prec, stream=stream) as dev:
-                    active = dev.set_megakernel(mode)
+                    active = dev.set_megakernel(mode) if mode is not None else False
                     for _ in range(3):
                         dev.run()
                     ms = timer.solves(dev.run, steps)

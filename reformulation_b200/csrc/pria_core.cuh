@@ -27,11 +27,11 @@
 //   one warp-level Michelot projection per column (theta <- (sum_{v>theta} v -
 //   1) / #{v > theta} to the fixed point, warp-shuffle sums), and writes the
 //   reflection r and the next step's combined x.
-// * y/z HALF-STEP: one thread-block CLUSTER per period block s.  Each warp
-//   projects y rows held in registers (Michelot, shuffles); the block's z
-//   values sit in the CTAs' shared memory and the z Michelot runs across the
-//   cluster, each round exchanging (sum, count) through distributed shared
-//   memory.  r is read once for both.
+// * y HALF-STEP: one warp per row, staged in shared memory (Michelot, shuffles).
+// * z HALF-STEP: one thread-block CLUSTER per period block s (or pair of them);
+//   the block's z values sit in the CTAs' shared memory and the Michelot runs
+//   across the cluster, each round exchanging (sum, count) through distributed
+//   shared memory.  Blocks that fit one CTA share a launch with y (yz_kernel).
 // * x, y, z hold the NEXT step's Halpern-combined point (as PRAQ's dual), so a
 //   reflected step streams x, x0, h, y, z (x kernel) and y, y0, z, z0, r (y/z
 //   kernel) and writes x, r, y, z: 14 ND reals per iteration.
