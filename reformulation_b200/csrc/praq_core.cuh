@@ -2237,12 +2237,14 @@ struct Solver final : SolverBase {
     template <bool W, bool P>
     cudaError_t enqueue_steps() {
         const int op = int(p.op_steps);
+        // With no edges a node step follows a node step, whose x it reads before
+        // its wait: plain launches then.
         for (int s = 0; s < op; ++s) {
             if (s + 1 < op) {
-                RB_TIMED(0, RB_CUDA_TRY(launch_pdl(node_kernel<Real, true, false, W, P>, nb_node, kBlock, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, 0)));
+                RB_TIMED(0, RB_CUDA_TRY(launch_ex(node_kernel<Real, true, false, W, P>, nb_node, kBlock, 0, m > 0, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, 0)));
                 if (m) RB_TIMED(1, RB_CUDA_TRY(launch_pdl(edge_plain_kernel<Real, P>, P ? nb_edge_pull : nb_edge_push, kBlock, stream, d, (const Real*)nullptr, s, 0, 0)));
             } else {
-                RB_TIMED(2, RB_CUDA_TRY(launch_pdl(node_kernel<Real, true, true, W, P>, nb_node, kBlock, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, 0)));
+                RB_TIMED(2, RB_CUDA_TRY(launch_ex(node_kernel<Real, true, true, W, P>, nb_node, kBlock, 0, m > 0, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, 0)));
                 if (m) RB_TIMED(3, RB_CUDA_TRY(launch_pdl(edge_kernel<Real, true, true, P>, nb_edge, kBlock, stream, d, (const Real*)nullptr, s, 0, 0)));
             }
         }

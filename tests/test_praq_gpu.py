@@ -540,6 +540,31 @@ def test_cluster_form_equals_graph(native, use_float32, case):
         assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
 
 
+@pytest.mark.parametrize("use_float32", [0, 1])
+def test_edgeless_on_the_graph(native, use_float32):
+    """Without edges the graph's node steps follow one another directly; each
+    must see the one before it complete.  The optimum is sum min(d, 0), the
+    launched and the replayed runs agree bit for bit, and with the grid form."""
+    from reformulation_b200.praq import DeviceSolver, Library
+    rng = np.random.default_rng(4)
+    n = 60_001
+    none = np.zeros(0, np.int64)
+    inst = QuboInstance("e", "e", n, rng.integers(-100, 101, n).astype(float), none, none, np.zeros(0))
+    p = Library().parameters(tolerance=1e-4 if use_float32 else 1e-8, use_float32=use_float32, max_iter=200_000)
+    out = []
+    for mode in (0, 2):
+        with DeviceSolver(inst, p) as dev:
+            assert dev.set_megakernel(mode) == (0 if mode == 0 else 1)
+            for _ in range(3):
+                assert dev.run() == 0
+                out.append(dev.result())
+    opt = np.minimum(inst.diag, 0.0).sum()
+    for r in out:
+        assert (r.iterations, r.lower, r.upper) == (out[0].iterations, out[0].lower, out[0].upper)
+        assert np.array_equal(r.x, out[0].x)
+    assert rel(out[0].upper, opt) <= 2 * p.tolerance
+
+
 def test_persistent_kernel_choice_and_edgeless(native):
     from reformulation_b200.instances import qubo_uniform_edges
     from reformulation_b200.praq import DeviceSolver, Library
