@@ -680,3 +680,37 @@ def test_convergence_trace_ring_wraps(native):
         dev.run()
         assert len(dev.trace()) == 0
     assert len(full) > 3 and last.tobytes() == full[-3:].tobytes()
+
+
+@pytest.mark.parametrize("use_float32", [0, 1])
+@pytest.mark.parametrize("form,n,m", [("single-cta", 700, 2800), ("cluster", 1500, 6000)])
+@pytest.mark.parametrize("op_steps", [2, 16, 300])
+def test_budget_of_a_whole_solve_launch(native, use_float32, form, n, m, op_steps):
+    """The forms that run many check blocks in one launch look at a wall-clock
+    budget at every check: a zero budget ends a solve that cannot converge
+    within two blocks, with the bracket of its last check, and one that is not
+    reached changes no bit of the result."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import DeviceSolver, Library
+    inst = qubo_uniform_edges(5, n, m)
+    lib = Library()
+    with DeviceSolver(inst, lib.parameters(tolerance=1e-15, max_iter=-1, use_float32=use_float32,
+                                           op_steps=op_steps)) as dev:
+        assert dev.set_megakernel(-1) == (2 if form == "single-cta" else 0)
+        dev.set_time_limit(0.0)
+        assert dev.run() == 2                          # PRAQ_STATUS_TIME_LIMIT
+        r = dev.result()
+        assert dev.launches() == 2                     # the start point and the solve: one of these forms
+        assert r.status == 2 and 0 < r.iterations <= 2 * op_steps
+        assert r.lower <= r.upper and np.all((r.x >= 0) & (r.x <= 1))
+    out = []
+    for mode, limit in ((-1, 1000.0), (0, -1.0)):
+        with DeviceSolver(inst, lib.parameters(tolerance=1e-4, max_iter=2400, use_float32=use_float32,
+                                               op_steps=op_steps)) as dev:
+            dev.set_megakernel(mode)
+            dev.set_time_limit(limit)
+            assert dev.run() in (0, 1)
+            out.append(dev.result(want_x=True, want_dual=True))
+    (a, ya), (b, yb) = out
+    assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
+    assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
