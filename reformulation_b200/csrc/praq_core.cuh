@@ -845,8 +845,37 @@ __device__ __forceinline__ void part_sums(const double (&v)[K], double* scratch,
     __syncthreads();
 }
 
-// A run of `v` added in order from zero, eight loads in flight (a value past
-// the end adds zero, which changes no sum's bits).
+// One long run, v[k .. e), added in order from zero by a whole warp: 32 lanes
+// load it coalesced, the next 128 values in flight while these are added, and
+// every lane adds every value in order.  (A value past the end adds zero, which
+// changes no sum's bits.)
+template <class Acc, class Real>
+__device__ __noinline__ Acc warp_long_run(const Real* v, int k, int e) {
+    constexpr int G = 4;
+    const int lane = threadIdx.x & 31;
+    Real t[G], nx[G];
+    auto load = [&](Real (&to)[G], int at) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const int q = at + 32 * g + lane;
+            to[g] = q < e ? v[q] : Real(0);
+        }
+    };
+    Acc s = Acc(0);
+    load(t, k);
+    for (; k < e; k += 32 * G) {
+        load(nx, k + 32 * G);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) s += Acc(__shfl_sync(0xffffffffu, t[g], j));
+            t[g] = nx[g];
+        }
+    }
+    return s;
+}
+
+// A run of `v` added in order from zero, eight loads in flight.
 template <class Acc, class Real>
 __device__ __forceinline__ Acc tiny_run(const int* ptr, const Real* v, int i, int m, int* status) {
     constexpr int U = 8;
@@ -863,17 +892,53 @@ __device__ __forceinline__ Acc tiny_run(const int* ptr, const Real* v, int i, in
     return s;
 }
 
+// The same for the nodes i of a warp (empty past the last node), where some run
+// of the instance may be long; all lanes call it.  One lane that adds a long
+// run holds the whole launch up (most in the cluster form, which reads these
+// runs from L2), so a warp with a few long runs adds them together, one after
+// the other.  Per solve with one node joined to every other, before this and
+// shared_long_run, now, and the graph, FP32 / FP64: n = 700, m = 1,700 (single
+// CTA) 0.97 / 1.84, 0.65 / 0.91, 0.85 / 1.45 ms; n = 2,000, m = 10,000 (cluster)
+// 18.8 / 22.4, 5.7 / 6.8, 6.4 / 11.6 ms.
+constexpr int kLongRun = 64, kLongLanes = 4;
+template <class Acc, class Real>
+__device__ __forceinline__ Acc tiny_runs(const int* ptr, const Real* v, int i, int n, int m, int* status) {
+    Acc s = Acc(0);
+    int k = 0, e = 0;
+    if (i < n) {
+        k = ptr[i];
+        e = ptr[i + 1];
+        if (!index_ok(0 <= k && k <= e && e <= m, status)) k = e = 0;
+    }
+    const unsigned longs = __ballot_sync(0xffffffffu, e - k > kLongRun);
+    const bool together = longs && __popc(longs) <= kLongLanes;
+    if (together) {
+        for (unsigned rest = longs; rest; rest &= rest - 1) {
+            const int owner = __ffs(rest) - 1;
+            const Acc all = warp_long_run<Acc>(v, __shfl_sync(0xffffffffu, k, owner), __shfl_sync(0xffffffffu, e, owner));
+            if (int(threadIdx.x & 31) == owner) s = all;
+        }
+    }
+    if (i < n && !(together && e - k > kLongRun)) s = tiny_run<Acc>(ptr, v, i, m, status);
+    return s;
+}
+
 // node_kernel_tile's step, term for term, one thread per node; the node tiles
 // kTinyParts at a time, dealt round-robin to the grid's CTAs (one in the
 // single-CTA form, the cluster's in the cluster form).
 template <class Real, bool Reflect, bool Check>
 __device__ __forceinline__ void tiny_node(const Dev<Real>& d, const Real* ys, const Real* yc, int step, int bounds_at_1,
-                                          int gate, int nb_node, double* scratch, double* qout) {
+                                          int gate, int nb_node, bool long_runs, double* scratch, double* qout) {
     const Control* c = d.ctl;
     if (skip(c, gate)) return;
     for (int base = int(blockIdx.x) * kTinyThreads; base < nb_node * kBlock; base += int(gridDim.x) * kTinyThreads) {
         const int i = base + int(threadIdx.x);
         double acc[kNodeSums] = {0.0, 0.0, 0.0};
+        Real s0 = Real(0), s1 = Real(0);
+        if (long_runs) {
+            s0 = tiny_runs<Real>(d.row_ptr, ys, i, d.n, d.m, &d.ctl->status);
+            s1 = tiny_runs<Real>(d.col_ptr, yc, i, d.n, d.m, &d.ctl->status);
+        }
         if (i < d.n) {
             const Real x2o = d.x2[i], di = d.diag[i], dg = d.deg[i];
             Real x1o = Real(0), x0o = Real(0);
@@ -881,8 +946,10 @@ __device__ __forceinline__ void tiny_node(const Dev<Real>& d, const Real* ys, co
                 x1o = d.x1[i];
                 x0o = d.x0[i];
             }
-            const Real s0 = tiny_run<Real>(d.row_ptr, ys, i, d.m, &d.ctl->status);
-            const Real s1 = tiny_run<Real>(d.col_ptr, yc, i, d.m, &d.ctl->status);
+            if (!long_runs) {
+                s0 = tiny_run<Real>(d.row_ptr, ys, i, d.m, &d.ctl->status);
+                s1 = tiny_run<Real>(d.col_ptr, yc, i, d.m, &d.ctl->status);
+            }
             const Real s = s0 + s1;
             Real x1v;
             if (Reflect) {
@@ -982,14 +1049,21 @@ __device__ __forceinline__ void tiny_edge(const Dev<Real>& d, const Real* ysrc, 
 // lower_kernel_tile's pass, term for term, one thread per node.
 template <class Real>
 __device__ __forceinline__ void tiny_lower(const Dev<Real>& d, const Real* ys, const Real* yc, int nb_node,
-                                           double* scratch, double* qout) {
+                                           bool long_runs, double* scratch, double* qout) {
     if (d.ctl->terminated) return;
     for (int base = int(blockIdx.x) * kTinyThreads; base < nb_node * kBlock; base += int(gridDim.x) * kTinyThreads) {
         const int i = base + int(threadIdx.x);
         double acc[1] = {0.0};
+        double s0 = 0.0, s1 = 0.0;
+        if (long_runs) {
+            s0 = tiny_runs<double>(d.row_ptr, ys, i, d.n, d.m, &d.ctl->status);
+            s1 = tiny_runs<double>(d.col_ptr, yc, i, d.n, d.m, &d.ctl->status);
+        }
         if (i < d.n) {
-            const double s0 = tiny_run<double>(d.row_ptr, ys, i, d.m, &d.ctl->status);
-            const double s1 = tiny_run<double>(d.col_ptr, yc, i, d.m, &d.ctl->status);
+            if (!long_runs) {
+                s0 = tiny_run<double>(d.row_ptr, ys, i, d.m, &d.ctl->status);
+                s1 = tiny_run<double>(d.col_ptr, yc, i, d.m, &d.ctl->status);
+            }
             const double s = s0 + s1;
             const double rc = double(d.diag[i]) - s;
             acc[0] = rc < 0.0 ? rc : 0.0;
@@ -1034,11 +1108,50 @@ __device__ __forceinline__ Real load_shared(unsigned at) {
 }
 
 // v[k .. e) added in order from zero; v in shared memory.  (A value past the
-// end adds zero, which changes no sum's bits.)
+// end adds zero, which changes no sum's bits.)  `long_runs`: some run of this
+// CTA's nodes has more than kLongRun values; all are then added in whole chunks
+// of 8, the next chunk's loads in flight while this one's values are added: a
+// hub's run is one thread's chain, which 4 values a pass with the end tested
+// for each made several times as long as its additions.  Out of line: its
+// registers are not the short runs' to pay for (inlined, n = 400, m = 2,000
+// took 0.24 against 0.22 ms in FP32).
 template <class Real>
-__device__ __forceinline__ Real shared_run(const Real* v, int k, int e) {
+__device__ __noinline__ Real shared_long_run(unsigned at, int count) {
+    constexpr int U = 8;
+    constexpr unsigned kBytes = unsigned(sizeof(Real));
+    Real s = Real(0), t[U];
+    if (count >= U) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) t[u] = load_shared<Real>(at + unsigned(u) * kBytes);
+        for (; count >= 2 * U; count -= U) {
+            at += U * kBytes;
+            Real nx[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) nx[u] = load_shared<Real>(at + unsigned(u) * kBytes);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                s += t[u];
+                t[u] = nx[u];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) s += t[u];
+        at += U * kBytes;
+        count -= U;
+    }
+    if (count > 0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) t[u] = load_shared<Real>(at + unsigned(min(u, count - 1)) * kBytes);
+#pragma unroll
+        for (int u = 0; u < U; ++u) s += u < count ? t[u] : Real(0);
+    }
+    return s;
+}
+template <class Real>
+__device__ __forceinline__ Real shared_run(const Real* v, int k, int e, bool long_runs) {
     constexpr int U = 4;
     const unsigned at = shared_address(v);
+    if (long_runs) return shared_long_run<Real>(at + unsigned(k) * unsigned(sizeof(Real)), e - k);
     Real s = Real(0);
     for (; k < e; k += U) {
         Real t[U];
@@ -1058,7 +1171,16 @@ struct TinyView {   // the instance and iterates in this CTA's shared memory
     const int *row_ptr, *col_ptr, *colpos;
     const int2* ends;
     int* status;
+    bool long_runs;
 };
+// Whether a run of the nodes [0, n) has more than kLongRun values; every thread
+// of the block calls it.
+__device__ __forceinline__ bool any_long_run(const int* row_ptr, const int* col_ptr, int n) {
+    int found = 0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        found |= row_ptr[i + 1] - row_ptr[i] > kLongRun || col_ptr[i + 1] - col_ptr[i] > kLongRun;
+    return __syncthreads_or(found) != 0;
+}
 
 template <class Real>
 __device__ __forceinline__ void tiny_node_plain(const TinyView<Real>& t, Real lw, Real rw, Real ps) {
@@ -1070,7 +1192,7 @@ __device__ __forceinline__ void tiny_node_plain(const TinyView<Real>& t, Real lw
         Real s = Real(0);
         if (i < t.n) {
             const int k = ptr[i], e = ptr[i + 1];
-            if (index_ok(0 <= k && k <= e && e <= t.m, t.status)) s = shared_run<Real>(v, k, e);
+            if (index_ok(0 <= k && k <= e && e <= t.m, t.status)) s = shared_run<Real>(v, k, e, t.long_runs);
         }
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         if (i < t.n && !half) {
@@ -1183,11 +1305,12 @@ tiny_solve_kernel(const __grid_constant__ Dev<Real> g, const __grid_constant__ P
     for (int i = threadIdx.x; i < nb_edge * kEdgeSums; i += blockDim.x)
         static_cast<double*>(at(L.pedge))[i] = 0.0;
     __syncthreads();
+    const bool long_runs = any_long_run(static_cast<const int*>(at(L.row_ptr)), static_cast<const int*>(at(L.col_ptr)), g.n);
     if (start) {
         // x1, y1 = _raw_step(x0, y0) with the bounds at the start point
         // (start_step's kernels), then the check before the loop
-        tiny_node<Real, false, true>(d, d.pred, d.pred1, 0, 1, 0, nb_node, scratch, qout);
-        tiny_lower<Real>(d, d.pred, d.pred1, nb_node, scratch, qout);
+        tiny_node<Real, false, true>(d, d.pred, d.pred1, 0, 1, 0, nb_node, long_runs, scratch, qout);
+        tiny_lower<Real>(d, d.pred, d.pred1, nb_node, long_runs, scratch, qout);
         __syncthreads();
         if (m) {
             tiny_edge<Real, false, true>(d, d.pred, 0, 1, 0, nb_edge, scratch, qout);
@@ -1214,6 +1337,7 @@ tiny_solve_kernel(const __grid_constant__ Dev<Real> g, const __grid_constant__ P
     view.colpos = static_cast<const int*>(at(L.colpos));
     view.ends = static_cast<const int2*>(at(L.ends));
     view.status = &d.ctl->status;
+    view.long_runs = long_runs;
     const int op = int(prm.op_steps);
     for (int b = 0; b < max_blocks && !d.ctl->terminated; ++b) {
         // one check block: enqueue_steps' kernels, in their order
@@ -1232,19 +1356,19 @@ tiny_solve_kernel(const __grid_constant__ Dev<Real> g, const __grid_constant__ P
             tiny_edge_plain<Real>(view, sw.lwn, sw.rwn, hs);
             __syncthreads();
         }
-        tiny_node<Real, true, true>(d, d.pred, d.pred1, op - 1, 0, 0, nb_node, scratch, qout);
+        tiny_node<Real, true, true>(d, d.pred, d.pred1, op - 1, 0, 0, nb_node, long_runs, scratch, qout);
         __syncthreads();
         if (m) {
             tiny_edge<Real, true, true>(d, nullptr, op - 1, 0, 0, nb_edge, scratch, qout);
             __syncthreads();
         }
-        tiny_lower<Real>(d, d.u2s, d.u2s1, nb_node, scratch, qout);
+        tiny_lower<Real>(d, d.u2s, d.u2s1, nb_node, long_runs, scratch, qout);
         __syncthreads();
         tiny_check(d.ctl, prm, d.scale, d.pnode, nb_node, d.pedge, nb_edge, d.plower, 1);
         if (threadIdx.x == 0) d.ctl->expired = globaltimer_ns() > deadline;
         __syncthreads();
         if (d.ctl->restart) {
-            tiny_node<Real, false, true>(d, d.u2s, d.u2s1, 0, 0, 1, nb_node, scratch, qout);
+            tiny_node<Real, false, true>(d, d.u2s, d.u2s1, 0, 0, 1, nb_node, long_runs, scratch, qout);
             __syncthreads();
             if (m) {
                 tiny_edge<Real, false, true>(d, d.u2s, 0, 0, 1, nb_edge, scratch, qout);
@@ -1444,6 +1568,8 @@ cluster_solve_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant_
         w[e] = d.w[e0 + e];
         dst[e] = cluster_address(pred1_at, q) + unsigned(pos - second_cut[q]) * unsigned(sizeof(Real));
     }
+    __syncthreads();
+    const bool long_runs = any_long_run(rp, cp, nodes);
     auto check = [&](int mode) {
         if (rank == 0) {
             tiny_check(d.ctl, prm, d.scale, d.pnode, nb_node, d.pedge, nb_edge, d.plower, mode);
@@ -1452,8 +1578,8 @@ cluster_solve_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant_
         cluster_barrier();
     };
     if (start) {   // the start step with the bounds at the start point, and the check before the loop
-        tiny_node<Real, false, true>(d, d.pred, d.pred1, 0, 1, 0, nb_node, scratch, qout);
-        tiny_lower<Real>(d, d.pred, d.pred1, nb_node, scratch, qout);
+        tiny_node<Real, false, true>(d, d.pred, d.pred1, 0, 1, 0, nb_node, true, scratch, qout);
+        tiny_lower<Real>(d, d.pred, d.pred1, nb_node, true, scratch, qout);
         cluster_barrier();
         tiny_edge<Real, false, true>(d, d.pred, 0, 1, 0, nb_edge, scratch, qout);
         cluster_barrier();
@@ -1491,7 +1617,7 @@ cluster_solve_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant_
                 for (int base = 0; base < nodes; base += kTinyThreads / 2) {
                     const int i = base + (tid >> 1);
                     Real sum = Real(0);
-                    if (i < nodes) sum = shared_run<Real>(v, ptr[i], ptr[i + 1]);
+                    if (i < nodes) sum = shared_run<Real>(v, ptr[i], ptr[i + 1], long_runs);
                     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
                     if (i < nodes) {   // (both threads of the pair compute it; one stores the point)
                         const Real x2o = x2[i], x1v = rfma(sw.lw, rfma(Real(2), x2o, -x1[i]), rmul(sw.rw, x0[i]));
@@ -1539,15 +1665,15 @@ cluster_solve_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant_
         for (int e = tid; e < edges; e += kTinyThreads) d.pred[e0 + e] = pred[e];
         for (int k = tid; k < seconds; k += kTinyThreads) d.pred1[k0 + k] = pred1[k];
         cluster_barrier();
-        tiny_node<Real, true, true>(d, d.pred, d.pred1, op - 1, 0, 0, nb_node, scratch, qout);
+        tiny_node<Real, true, true>(d, d.pred, d.pred1, op - 1, 0, 0, nb_node, true, scratch, qout);
         cluster_barrier();
         tiny_edge<Real, true, true>(d, nullptr, op - 1, 0, 0, nb_edge, scratch, qout);
         cluster_barrier();
-        tiny_lower<Real>(d, d.u2s, d.u2s1, nb_node, scratch, qout);
+        tiny_lower<Real>(d, d.u2s, d.u2s1, nb_node, true, scratch, qout);
         cluster_barrier();
         check(1);
         if (d.ctl->restart) {   // uniform over the cluster
-            tiny_node<Real, false, true>(d, d.u2s, d.u2s1, 0, 0, 1, nb_node, scratch, qout);
+            tiny_node<Real, false, true>(d, d.u2s, d.u2s1, 0, 0, 1, nb_node, true, scratch, qout);
             cluster_barrier();
             tiny_edge<Real, false, true>(d, d.u2s, 0, 0, 1, nb_edge, scratch, qout);
             cluster_barrier();

@@ -714,3 +714,80 @@ def test_budget_of_a_whole_solve_launch(native, use_float32, form, n, m, op_step
     (a, ya), (b, yb) = out
     assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
     assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
+
+
+def _star_instance(lengths, n, extra, spread, seed=8):
+    """Hubs with `lengths` leaves each, at low node numbers (first ends of
+    their edges) and, mirrored, at high ones (second ends); next to each other
+    or `spread` nodes apart, over uniform edges."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    rng = np.random.default_rng(seed)
+    code = []
+    for k, length in enumerate(lengths):
+        lo, hi = k * spread, n - 1 - k * spread
+        mid = np.arange(len(lengths) * spread, n - len(lengths) * spread)
+        code.append(lo * n + rng.choice(mid, length, replace=False))
+        code.append(rng.choice(mid, length, replace=False) * n + hi)
+    if extra:
+        rest = qubo_uniform_edges(seed, n, extra)
+        code.append(rest.rows * n + rest.cols)
+    code = np.unique(np.concatenate(code))
+    vals = rng.integers(1, 101, code.size) * rng.choice([-1.0, 1.0], code.size)
+    return QuboInstance("stars", "stars", n, rng.integers(-100, 101, n) * 1.0, code // n, code % n, vals)
+
+
+@pytest.mark.parametrize("use_float32", [0, 1])
+@pytest.mark.parametrize("form,spread", [("single-cta", 1), ("single-cta", 8), ("cluster", 1), ("cluster", 8)])
+def test_long_runs_equal_graph(native, use_float32, form, spread):
+    """Runs of every length at which the sums' chunks end (16, 24 and their
+    neighbours in the plain steps; 64, 128, 192 and theirs in the checks),
+    few and many of them in a warp, against the graph bit for bit."""
+    from reformulation_b200.praq import Library
+    lengths = [15, 16, 17, 23, 24, 25, 33, 63, 64, 65, 66, 127, 128, 129, 191, 193, 257]
+    inst = (_star_instance(lengths[::2], 520, 0, spread) if form == "single-cta" else
+            _star_instance(lengths, 1100, 4000, spread))
+    p = Library().parameters(tolerance=1e-12, use_float32=use_float32, max_iter=320)
+    (on, (a,), launches), (_, (b,), _) = (_praq_runs_any(inst, p, mode) for mode in (-1, 0))
+    assert on == (2 if form == "single-cta" else 0) and launches == 2
+    assert (a[0].iterations, a[0].lower, a[0].upper) == (b[0].iterations, b[0].lower, b[0].upper)
+    assert np.array_equal(a[0].x, b[0].x) and np.array_equal(a[1], b[1])
+
+
+def _praq_runs_any(inst, p, mode, runs=1):
+    from reformulation_b200.praq import DeviceSolver
+    out = []
+    with DeviceSolver(inst, p) as dev:
+        active = dev.set_megakernel(mode)
+        for _ in range(runs):
+            assert dev.run() in (0, 1)
+            out.append(dev.result(want_x=True, want_dual=True))
+        return active, out, dev.launches()
+
+
+@pytest.mark.parametrize("use_float32", [0, 1])
+@pytest.mark.parametrize("form,n,extra", [("single-cta", 700, 400), ("cluster", 2000, 8000)])
+def test_hub_is_not_slow(native, use_float32, form, n, extra):
+    """One node with an edge to every other: the forms the solver takes by
+    itself are not behind the graph's kernels there (they were, by 1.2 to 3
+    times, while one thread added the hub's run a few values at a time)."""
+    import time
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import DeviceSolver, Library
+    rest = qubo_uniform_edges(3, n, extra)
+    keep = rest.rows > 0
+    rows = np.concatenate([np.zeros(n - 1, np.int64), rest.rows[keep]])
+    cols = np.concatenate([np.arange(1, n), rest.cols[keep]])
+    inst = QuboInstance("hub", "hub", n, rest.diag, rows, cols,
+                        np.random.default_rng(2).integers(1, 100, rows.size) * 1.0)
+    best = {}
+    for mode in (-1, 0):
+        with DeviceSolver(inst, Library().parameters(tolerance=1e-15, max_iter=64, use_float32=use_float32)) as dev:
+            active = dev.set_megakernel(mode)
+            best[mode] = float("inf")
+            for _ in range(8):
+                start = time.perf_counter()
+                dev.run()
+                best[mode] = min(best[mode], time.perf_counter() - start)
+            if mode == -1:
+                assert active == (2 if form == "single-cta" else 0) and dev.launches() == 2
+    assert best[-1] <= 1.1 * best[0]
