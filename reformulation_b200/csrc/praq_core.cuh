@@ -359,6 +359,14 @@ template <class Real, bool Reflect, bool Check, bool Wide = false, bool Pull = f
 __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, const Real* ys, const Real* yc, int step,
                                                  int bounds_at_1, int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
+    // Ahead of the wait only in a chain, and only where the step is sure to be
+    // taken: a gated (restart) step leaves in most blocks, a finished instance
+    // of a batch in all.
+    const bool early = reads_early<Wait>() && (Reflect || !gate);
+    if (!early) {
+        wait();
+        if (skip(c, gate)) return;
+    }
     __shared__ double scratch[kNodeSums * 32];
     Real* stage = warp_stage<Real, stage_runs<Wide>()>();
     const int lane = threadIdx.x & 31;
@@ -378,8 +386,10 @@ __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, c
             x0o = d.x0[i];
         }
     }
-    wait();
-    if (skip(c, gate)) return;
+    if (early) {
+        wait();
+        if (skip(c, gate)) return;
+    }
     const Real s = scatter_at<Real, Real, Wide, Pull>(d, first, second, ys, yc, lane, stage);
     double acc[kNodeSums] = {0.0, 0.0, 0.0};
     if (owner) {
@@ -428,11 +438,16 @@ template <class Real, bool Reflect, bool Check, bool Pull = false, int EPT = kEd
 __device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, const Real* ysrc, int step, int bounds_at_1,
                                                  int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    __shared__ double scratch[kEdgeSums * 32];
-    const int base = tile * (kBlock * EPT) + threadIdx.x;
-    // the edges' constants, their dual and anchor, the control block: nothing
+    const bool early = reads_early<Wait>() && (Reflect || !gate);   // (as in the node half)
+    // the control block, the edges' constants, their dual and anchor: nothing
     // the kernel ahead (the node half) writes
     const bool off = skip(c, gate);
+    if (!early) {
+        wait();
+        if (off) return;
+    }
+    __shared__ double scratch[kEdgeSums * 32];
+    const int base = tile * (kBlock * EPT) + threadIdx.x;
     const Real hs = Real(0.5 * kEta * c->omega);
     const double kn = Reflect ? double(c->restart_iter + step + 2) : 1.0;
     const Real lwn = Real(kn / (kn + 1.0)), rwn = Real(1.0 / (kn + 1.0));
@@ -450,8 +465,10 @@ __device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, c
             at1[t] = Pull ? e : d.colpos[e];
         }
     }
-    wait();
-    if (off) return;
+    if (early) {
+        wait();
+        if (off) return;
+    }
     Real ri[EPT], rj[EPT];
 #pragma unroll
     for (int t = 0; t < EPT; ++t) {
@@ -527,6 +544,11 @@ edge_plain_kernel(Dev<Real> d, const Real* ysrc, int step, int bounds_at_1, int 
 template <class Real, bool Wide = false, bool Pull = false, class Wait = NoWait>
 __device__ __forceinline__ void lower_kernel_tile(const Dev<Real>& d, int tile, const Real* ys, const Real* yc,
                                                   Wait wait = Wait()) {
+    constexpr bool early = reads_early<Wait>();
+    if (!early) {
+        wait();
+        if (d.ctl->terminated) return;
+    }
     __shared__ double scratch[32];
     Real* stage = warp_stage<Real, stage_runs<Wide>()>();
     const int lane = threadIdx.x & 31;
@@ -534,8 +556,10 @@ __device__ __forceinline__ void lower_kernel_tile(const Dev<Real>& d, int tile, 
     const long long i = base + lane;
     const RunBounds first = run_bounds(d.row_ptr, d.n, base, lane), second = run_bounds(d.col_ptr, d.n, base, lane);
     const Real di = i < d.n ? d.diag[i] : Real(0);
-    wait();
-    if (d.ctl->terminated) return;
+    if (early) {
+        wait();
+        if (d.ctl->terminated) return;
+    }
     const double s = scatter_at<Real, double, Wide, Pull>(d, first, second, ys, yc, lane, stage);
     double acc[1] = {0.0};
     if (i < d.n) {
@@ -676,7 +700,7 @@ template <class Real, bool Reflect, bool Check, bool Wide>
 __device__ __forceinline__ void mega_node(const Dev<Real>& d, const MegaArgs& a, const Real* ys, const Real* yc,
                                           int step, int gate, int bounds_at_1 = 0) {
     for (int t = int(blockIdx.x); t < a.nb_node; t += gridDim.x) {
-        node_kernel_tile<Real, Reflect, Check, Wide, false>(d, t, ys, yc, step, bounds_at_1, gate);
+        node_kernel_tile<Real, Reflect, Check, Wide, false>(d, t, ys, yc, step, bounds_at_1, gate, InLaunch());
         __syncthreads();   // the next tile reuses the staging buffer
     }
 }
@@ -685,7 +709,7 @@ template <class Real, bool Reflect, bool Check>
 __device__ __forceinline__ void mega_edge(const Dev<Real>& d, const MegaArgs& a, const Real* ysrc, int step,
                                           int gate, int bounds_at_1 = 0) {
     for (int t = int(blockIdx.x); t < a.nb_edge; t += gridDim.x) {
-        edge_kernel_tile<Real, Reflect, Check, false>(d, t, ysrc, step, bounds_at_1, gate);
+        edge_kernel_tile<Real, Reflect, Check, false, kEdgesPerThread>(d, t, ysrc, step, bounds_at_1, gate, InLaunch());
         __syncthreads();
     }
 }
@@ -693,7 +717,7 @@ __device__ __forceinline__ void mega_edge(const Dev<Real>& d, const MegaArgs& a,
 template <class Real, bool Wide>
 __device__ __forceinline__ void mega_lower(const Dev<Real>& d, const MegaArgs& a, const Real* ys, const Real* yc) {
     for (int t = int(blockIdx.x); t < a.nb_node; t += gridDim.x) {
-        lower_kernel_tile<Real, Wide, false>(d, t, ys, yc);
+        lower_kernel_tile<Real, Wide, false>(d, t, ys, yc, InLaunch());
         __syncthreads();
     }
 }
@@ -750,6 +774,7 @@ cudaError_t grid_capacity(Fn fn, int* out) {
 template <class Real, bool Wide>
 __global__ void __launch_bounds__(kBlock, 1)
 mega_block_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant__ Params prm, MegaArgs a) {
+    if (d.ctl->terminated) return;   // the block queued behind the last one (uniform: written by an earlier launch)
     auto sync = [&]() {
         if (grid_sync(a.bar, a.expect, a.wait_ns)) return true;
         if (threadIdx.x == 0) d.ctl->status = kMegaWaitStatus;

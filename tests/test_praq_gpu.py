@@ -791,3 +791,19 @@ def test_hub_is_not_slow(native, use_float32, form, n, extra):
             if mode == -1:
                 assert active == (2 if form == "single-cta" else 0) and dev.launches() == 2
     assert best[-1] <= 1.1 * best[0]
+
+
+def test_gated_step_leaves_before_it_reads(native):
+    """The restart step's launches in a block that does not restart read no
+    edge: a fraction of a step's time (here 0.23; 0.53 while they read the
+    instance before they looked whether to)."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import DeviceSolver, Library
+    inst = qubo_uniform_edges(2, 400_000, 4_000_000)
+    p = Library().parameters(tolerance=1e-14, max_iter=160, use_float32=1, beta_sufficient=1e-300,
+                             beta_necessary=1e-300, beta_artificial=1e9)   # no restart
+    with DeviceSolver(inst, p) as dev:
+        dev.run()
+        _, kinds = dev.run_profiled()
+    step, restart = (kinds[k][0] / kinds[k][1] for k in ("edge", "restart_edge"))
+    assert restart <= 0.38 * step
