@@ -119,17 +119,22 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // does not enter, so its steps read before they decide (n = 12,000, m = 150,000
 // in the grid form: 2 % faster a solve than deciding first).
 struct NoWait {
+    static constexpr bool kReadsEarly = false;
     __device__ __forceinline__ void operator()() const {}
 };
-struct InLaunch : NoWait {};
+struct InLaunch : NoWait {
+    static constexpr bool kReadsEarly = true;
+};
 struct PdlWait {
+    static constexpr bool kReadsEarly = true;
     __device__ __forceinline__ void operator()() const {
         pdl_wait();
         pdl_launch_dependents();
     }
 };
-template <class Wait>
-constexpr bool reads_early() { return !std::is_same_v<Wait, NoWait>; }
+struct PdlWaitFirst : PdlWait {   // waits and decides, then reads
+    static constexpr bool kReadsEarly = false;
+};
 
 // Launch `kernel` on `stream` with `smem` bytes of dynamic shared memory and, if
 // `pdl`, with the programmatic stream-serialization attribute (the kernel must

@@ -362,7 +362,7 @@ __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, c
     // Ahead of the wait only in a chain, and only where the step is sure to be
     // taken: a gated (restart) step leaves in most blocks, a finished instance
     // of a batch in all.
-    const bool early = reads_early<Wait>() && (Reflect || !gate);
+    const bool early = Wait::kReadsEarly && (Reflect || !gate);
     if (!early) {
         wait();
         if (skip(c, gate)) return;
@@ -438,7 +438,7 @@ template <class Real, bool Reflect, bool Check, bool Pull = false, int EPT = kEd
 __device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, const Real* ysrc, int step, int bounds_at_1,
                                                  int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    const bool early = reads_early<Wait>() && (Reflect || !gate);   // (as in the node half)
+    const bool early = Wait::kReadsEarly && (Reflect || !gate);   // (as in the node half)
     // the control block, the edges' constants, their dual and anchor: nothing
     // the kernel ahead (the node half) writes
     const bool off = skip(c, gate);
@@ -521,10 +521,10 @@ __device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, c
     }
 }
 
-template <class Real, bool Reflect, bool Check, bool Pull = false>
+template <class Real, bool Reflect, bool Check, bool Pull = false, class Wait = PdlWait>
 __global__ void __launch_bounds__(kBlock)
 edge_kernel(Dev<Real> d, const Real* ysrc, int step, int bounds_at_1, int gate) {
-    edge_kernel_tile<Real, Reflect, Check, Pull, kEdgesPerThread>(d, blockIdx.x, ysrc, step, bounds_at_1, gate, PdlWait());
+    edge_kernel_tile<Real, Reflect, Check, Pull, kEdgesPerThread>(d, blockIdx.x, ysrc, step, bounds_at_1, gate, Wait());
 }
 
 // The reflected step without check sums, on its own grid (tiles of kBlock *
@@ -532,11 +532,11 @@ edge_kernel(Dev<Real> d, const Real* ysrc, int step, int bounds_at_1, int gate) 
 // more registers, so the CTAs an SM holds are pinned: FP64 4 (3 unpinned: 6.36
 // against 6.22 ms a solve at n = 4e5, m = 4e6), FP32 pull 5 (6: 27.3 against
 // 26.4 ms at n = 2e6, m = 2e7), FP32 push 8.
-template <class Real, bool Pull = false>
+template <class Real, bool Pull = false, class Wait = PdlWait>
 __global__ void __launch_bounds__(kBlock, sizeof(Real) == 8 ? 4 : Pull ? 5 : 8)
 edge_plain_kernel(Dev<Real> d, const Real* ysrc, int step, int bounds_at_1, int gate) {
     edge_kernel_tile<Real, true, false, Pull, plain_edges_per_thread<Real, Pull>()>(d, blockIdx.x, ysrc, step, bounds_at_1,
-                                                                                  gate, PdlWait());
+                                                                                  gate, Wait());
 }
 
 // The node part of the lower bound, sum_i min(d_i - (S^T y)_i, 0), at the
@@ -544,7 +544,7 @@ edge_plain_kernel(Dev<Real> d, const Real* ysrc, int step, int bounds_at_1, int 
 template <class Real, bool Wide = false, bool Pull = false, class Wait = NoWait>
 __device__ __forceinline__ void lower_kernel_tile(const Dev<Real>& d, int tile, const Real* ys, const Real* yc,
                                                   Wait wait = Wait()) {
-    constexpr bool early = reads_early<Wait>();
+    constexpr bool early = Wait::kReadsEarly;
     if (!early) {
         wait();
         if (d.ctl->terminated) return;
@@ -1939,6 +1939,7 @@ struct Solver final : SolverBase {
     int nb_node = 1, nb_edge = 1, nb_edge_push = 1, nb_edge_pull = 1;
     bool wide = false;   // node gather of both runs at once (warp_runs2)
     bool pull = false;   // slot-1 layout (see the layout notes at the top)
+    bool edges_wait = false;   // FP64 push: the edge half waits before it reads
     bool allow_pull = true;   // false: always push (the batched engine's kernels)
     bool allow_mega = true;   // false: never the persistent kernel (the batched engine's instances)
     cudaGraph_t graph = nullptr;
@@ -2004,6 +2005,15 @@ struct Solver final : SolverBase {
         if (!mirror) return PRAQ_ERROR_CUDA;
         std::memset(static_cast<void*>(mirror), 0, sizeof(Control));   // no run yet: no trace, nothing done
         pull = choose_pull(in.m);
+        // The edge half's reads ahead of its wait run beside the node half's last
+        // CTAs.  In FP64 they hold a register more than its 64, and once the edge
+        // arrays exceed L2 the half is bound by DRAM and gains nothing from them:
+        // per solve, reading ahead against waiting first, m = 2.0M (88 MB) 6.81
+        // against 6.86 ms, 2.5M 7.50 against 7.45, 3M (132 MB, the L2 size) 9.67
+        // against 9.71, 4M 13.58 against 13.27, 5.5M 20.43 against 19.81.  (FP32
+        // push, and both in the pull layout: 0.3 to 4 % faster reading ahead; FP64
+        // pull at m = 8M 0.8 % slower, at 20M 0.9 % faster.)
+        edges_wait = sizeof(Real) == 8 && !pull && edge_bytes(in.m) > l2_bytes();
         const int st = layout(in);
         if (st) return st;
         nb_node = ceil_div(n, kBlock);   // one node per thread
@@ -2412,10 +2422,13 @@ struct Solver final : SolverBase {
             return cudaMemcpyAsync(mirror, d.ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream);
         }
         if (pull) return wide ? enqueue_steps<true, true>() : enqueue_steps<false, true>();
+        if constexpr (sizeof(Real) == 8) {
+            if (edges_wait) return wide ? enqueue_steps<true, false, PdlWaitFirst>() : enqueue_steps<false, false, PdlWaitFirst>();
+        }
         return wide ? enqueue_steps<true, false>() : enqueue_steps<false, false>();
     }
 
-    template <bool W, bool P>
+    template <bool W, bool P, class EdgeWait = PdlWait>
     cudaError_t enqueue_steps() {
         const int op = int(p.op_steps);
         // With no edges a node step follows a node step, whose x it reads before
@@ -2423,10 +2436,10 @@ struct Solver final : SolverBase {
         for (int s = 0; s < op; ++s) {
             if (s + 1 < op) {
                 RB_TIMED(0, RB_CUDA_TRY(launch_ex(node_kernel<Real, true, false, W, P>, nb_node, kBlock, 0, m > 0, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, 0)));
-                if (m) RB_TIMED(1, RB_CUDA_TRY(launch_pdl(edge_plain_kernel<Real, P>, P ? nb_edge_pull : nb_edge_push, kBlock, stream, d, (const Real*)nullptr, s, 0, 0)));
+                if (m) RB_TIMED(1, RB_CUDA_TRY(launch_pdl(edge_plain_kernel<Real, P, EdgeWait>, P ? nb_edge_pull : nb_edge_push, kBlock, stream, d, (const Real*)nullptr, s, 0, 0)));
             } else {
                 RB_TIMED(2, RB_CUDA_TRY(launch_ex(node_kernel<Real, true, true, W, P>, nb_node, kBlock, 0, m > 0, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, 0)));
-                if (m) RB_TIMED(3, RB_CUDA_TRY(launch_pdl(edge_kernel<Real, true, true, P>, nb_edge, kBlock, stream, d, (const Real*)nullptr, s, 0, 0)));
+                if (m) RB_TIMED(3, RB_CUDA_TRY(launch_pdl(edge_kernel<Real, true, true, P, EdgeWait>, nb_edge, kBlock, stream, d, (const Real*)nullptr, s, 0, 0)));
             }
         }
         RB_TIMED(4, RB_CUDA_TRY(launch_pdl(lower_kernel<Real, W, P>, nb_node, kBlock, stream, d, (const Real*)d.u2s, (const Real*)d.u2s1)));
@@ -2540,14 +2553,19 @@ struct Solver final : SolverBase {
         if (env && !std::strcmp(env, "push")) return false;
         if (env && !std::strcmp(env, "pull")) return true;
         if (kPull != 2) return kPull == 1;
+        const double l2 = l2_bytes();
+        return l2 > 0.0 && edge_bytes(m_) > 2.0 * l2;
+    }
+    // the step's edge arrays (ends, w, pred, pred1, u0 and the index), and L2 (0: unknown)
+    static double edge_bytes(int64_t m_) { return double(m_) * (12.0 + 4.0 * sizeof(Real)); }
+    static double l2_bytes() {
         int l2 = 0;
-        if (once_per_device(&l2, [](int* v) {
-                int dev = 0;
-                RB_CUDA_TRY(cudaGetDevice(&dev));
-                return cudaDeviceGetAttribute(v, cudaDevAttrL2CacheSize, dev);
-            }) != cudaSuccess)
-            return false;
-        return double(m_) * (12.0 + 4.0 * sizeof(Real)) > 2.0 * double(l2);
+        const cudaError_t st = once_per_device(&l2, [](int* v) {
+            int dev = 0;
+            RB_CUDA_TRY(cudaGetDevice(&dev));
+            return cudaDeviceGetAttribute(v, cudaDevAttrL2CacheSize, dev);
+        });
+        return st == cudaSuccess ? double(l2) : 0.0;
     }
 
     // Cold (or warm) start, the first vanilla step and the check before the loop.

@@ -807,3 +807,20 @@ def test_gated_step_leaves_before_it_reads(native):
         _, kinds = dev.run_profiled()
     step, restart = (kinds[k][0] / kinds[k][1] for k in ("edge", "restart_edge"))
     assert restart <= 0.38 * step
+
+
+@pytest.mark.parametrize("m", [2_990_003, 3_100_001])
+def test_fp64_push_beyond_l2_equals_grid_form(native, m):
+    """FP64 in the push layout, the edge arrays (44 bytes an edge) below and
+    above the L2 size, where the edge half waits before it reads: launched
+    and replayed runs agree bit for bit with each other and the grid form."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import Library
+    inst = qubo_uniform_edges(3, 250_007, m)
+    p = Library().parameters(tolerance=1e-12, max_iter=64)
+    (_, graph, _), (on, grid, _) = (_praq_runs_any(inst, p, mode, runs=2) for mode in (0, 2))
+    assert on == 1
+    for a, ya in graph[1:] + grid:
+        b, yb = graph[0]
+        assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
+        assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
