@@ -1964,6 +1964,9 @@ struct Solver final : SolverBase {
     bool tiny = false, tiny_fits = false;
     size_t tiny_smem = 0;
     static constexpr int kTinyBlocks = 128;
+    // edge bytes of a check block from which a first run waits for each check
+    static constexpr double kLongBlockBytes = 400e6;
+    static constexpr int kWaitedChecks = 10;
     // The cluster form (cluster_solve_kernel): CTAs of its cluster (0: the
     // instance does not take it), its cut and dynamic shared memory.
     bool clustered = false;
@@ -2602,14 +2605,17 @@ struct Solver final : SolverBase {
             const int st = start_solve();
             if (st) return st;
         }
-        // Keep one block in flight ahead of the one being inspected; blocks
-        // launched after termination see the flag and return at once.  A first
-        // run of the pull layout, whose blocks take milliseconds, waits for each
-        // check instead: its kernels read what they may before they see the
-        // flag, and the block too many costs 1.2 ms at n = 2e6, m = 2e7, five
-        // waits a tenth of that.  (A replayed block behind the end runs its gate
-        // alone.)
-        const int depth = pull && !exec && !mega ? 1 : 2;
+        // Keep one block in flight ahead of the one being inspected.  A replayed
+        // block behind the end runs its gate alone, but a first run's, launched
+        // kernel by kernel, reads what it may before it sees the flag.  So a
+        // first run of long blocks waits for each check instead, which costs some
+        // 5 us a check; after kWaitedChecks of them it queues ahead too.  First
+        // runs, queued ahead against waiting, FP32 / FP64: n = 1e5, m = 1e6 1.43
+        // against 1.37 / 3.25 against 3.19 ms; 4e5, 4e6 5.56 against 5.31 / 13.34
+        // against 13.24; 2e6, 2e7 (pull) FP32 28.1 against 27.6; with many checks
+        // (2e5, 8e5 FP64) 7.76 against 7.82.
+        const bool waits = !exec && !mega && double(p.op_steps) * edge_bytes(m) >= kLongBlockBytes;
+        int depth = waits ? 1 : 2, waited = 0;
         if (!mirror->terminated) {
             for (int k = 0; k < depth; ++k) {
                 if (launch_block() != cudaSuccess) return PRAQ_ERROR_CUDA;
@@ -2631,7 +2637,14 @@ struct Solver final : SolverBase {
                 if (launch_block() != cudaSuccess) return PRAQ_ERROR_CUDA;
                 if (cudaEventRecord(done[k], stream) != cudaSuccess) return PRAQ_ERROR_CUDA;
                 nlaunch += block_launches();
-                k = (k + 1) % depth;
+                if (depth == 1 && ++waited == kWaitedChecks) {
+                    depth = 2;
+                    if (launch_block() != cudaSuccess) return PRAQ_ERROR_CUDA;
+                    if (cudaEventRecord(done[1], stream) != cudaSuccess) return PRAQ_ERROR_CUDA;
+                    nlaunch += block_launches();
+                } else {
+                    k = (k + 1) % depth;
+                }
             }
         }
         if (cudaMemcpyAsync(mirror, d.ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||

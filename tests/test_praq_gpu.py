@@ -824,3 +824,24 @@ def test_fp64_push_beyond_l2_equals_grid_form(native, m):
         b, yb = graph[0]
         assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
         assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
+
+
+@pytest.mark.parametrize("checks", [3, 10, 11, 12, 17])
+def test_first_run_of_long_blocks(native, checks):
+    """A first run of long check blocks waits for its first ten checks and
+    queues a block ahead from then on: it ends where a repeated run does."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import DeviceSolver, Library
+    inst = qubo_uniform_edges(4, 100_000, 1_000_000)
+    with DeviceSolver(inst, Library().parameters(tolerance=1e-15, max_iter=16 * checks, use_float32=1,
+                                                 op_steps=16)) as dev:
+        out = []
+        for _ in range(2):
+            assert dev.run() == 1                      # the iteration limit
+            out.append((dev.result(want_x=True, want_dual=True), dev.launches()))
+    ((a, ya), la), ((b, yb), lb) = out
+    assert a.iterations == 16 * checks
+    assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
+    assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
+    block = 2 * 16 + 5                                 # its launches
+    assert la == 5 + block * (checks + (checks > 10))
