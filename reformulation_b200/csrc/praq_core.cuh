@@ -1422,7 +1422,7 @@ tiny_solve_kernel(const __grid_constant__ Dev<Real> g, const __grid_constant__ P
 // of work.  cluster_solve_kernel runs the solve in ONE thread-block cluster of
 // up to kClusterMax CTAs of kTinyThreads, the instance spread over their
 // shared memories:
-// * a CTA owns a range of nodes (cut so that the bytes balance), the first-end
+// * a CTA owns a range of nodes (cut so that the work balances), the first-end
 //   edges of those nodes (one range of the sorted edges) and their slot-1
 //   values (one range of second-end order);
 // * every CTA holds a copy of the whole reflection r, written by the nodes'
@@ -1475,22 +1475,30 @@ __host__ __device__ inline ClusterLayout cluster_layout(int n, int nodes, int ed
     return t;
 }
 
-// Cut q of `parts`: the first node at which the bytes before it (a monotone
-// sum of run pointers) reach q shares of the total.
+// Cut q of `parts`: the first node at which the work before it (a monotone sum
+// of run pointers) reaches q shares of the total.  An edge's work is its bytes;
+// a node and a slot-1 value count kCutWeight times theirs (a node is two
+// threads' step and 15 remote stores, a slot-1 value is added in a chain): cut
+// by bytes alone, the last CTAs, whose nodes have few first-end edges, held so
+// many nodes that the others waited for them.  Per solve by bytes, with the
+// weight, and the graph: n = 2,000, m = 12,000 FP32 0.63, 0.51, 0.56 ms; 1,500,
+// 9,000 0.51, 0.495, 0.55; FP64 3,000, 24,000 1.16, 0.96, 1.08; 2,000, 12,000
+// 0.96, 0.87, 1.15 (2: 0.94; 3: 0.88; 6: 0.89).
+constexpr int kCutWeight = 4;
 __global__ void cluster_plan_kernel(int n, int m, int parts, int real, const int* __restrict__ row_ptr,
                                     const int* __restrict__ col_ptr, ClusterPlan* plan) {
     __shared__ int node[kClusterMax + 1];
     const int q = threadIdx.x;
-    auto bytes = [&](int i) {
-        return (long long)cluster_edge_bytes(real) * row_ptr[i] + (long long)real * col_ptr[i] +
-               (long long)cluster_node_bytes(real) * i;
+    auto work = [&](int i) {
+        return (long long)cluster_edge_bytes(real) * row_ptr[i] +
+               kCutWeight * ((long long)real * col_ptr[i] + (long long)cluster_node_bytes(real) * i);
     };
     if (q <= parts) {
-        const long long want = bytes(n) * q / parts;
+        const long long want = work(n) * q / parts;
         int lo = 0, hi = n;
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (bytes(mid) < want) lo = mid + 1; else hi = mid;
+            if (work(mid) < want) lo = mid + 1; else hi = mid;
         }
         node[q] = q == parts ? n : lo & ~3;   // a CTA's part of r starts on 16 bytes
     }

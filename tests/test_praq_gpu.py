@@ -845,3 +845,24 @@ def test_first_run_of_long_blocks(native, checks):
     assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
     block = 2 * 16 + 5                                 # its launches
     assert la == 5 + block * (checks + (checks > 10))
+
+
+@pytest.mark.parametrize("use_float32,n,m", [(1, 2000, 12_000), (1, 2048, 12_288), (0, 3000, 24_000), (0, 3072, 24_576)])
+def test_cluster_is_not_behind_the_graph_at_its_bound(native, use_float32, n, m):
+    """The largest instances the cluster form takes by itself: not slower than
+    the graph's kernels (by 3 to 14 % while the cut evened bytes)."""
+    import time
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import DeviceSolver, Library
+    inst = qubo_uniform_edges(2, n, m)
+    best = {}
+    for mode in (-1, 0):
+        with DeviceSolver(inst, Library().parameters(tolerance=1e-15, max_iter=160, use_float32=use_float32)) as dev:
+            dev.set_megakernel(mode)
+            best[mode] = float("inf")
+            for _ in range(12):
+                start = time.perf_counter()
+                dev.run()
+                best[mode] = min(best[mode], time.perf_counter() - start)
+            assert mode == 0 or dev.launches() == 2
+    assert best[-1] <= 1.01 * best[0]
