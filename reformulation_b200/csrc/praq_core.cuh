@@ -2109,13 +2109,12 @@ struct Solver final : SolverBase {
                 RB_CUDA_TRY(cudaGetDevice(&dev));
                 RB_CUDA_TRY(cudaFuncGetAttributes(&fa, tiny_solve_kernel<Real>));
                 RB_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-                *v = optin > int(fa.sharedSizeBytes) ? optin - int(fa.sharedSizeBytes) : 0;
+                *v = std::max(0, optin - int((fa.sharedSizeBytes + 15) / 16 * 16));   // (dynamic memory starts on 16 bytes)
                 return cudaFuncSetAttribute(tiny_solve_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, *v);
             }));
             tiny_smem = tiny_layout(n, m, nb_node, nb_edge, int(sizeof(Real))).total;
-            // check_body's row reductions keep the 256-thread order up to 256 rows
-            tiny_fits = tiny_smem <= size_t(room) && nb_node <= kBlock && nb_edge <= kBlock;
-            if (!tiny_fits) RB_CUDA_TRY(init_cluster());
+            tiny_fits = tiny_smem <= size_t(room);
+            if (!tiny_fits || step_work() > kTinyWork) RB_CUDA_TRY(init_cluster());
         }
         // REFORM_PRAQ_MEGA=0|1 sets the initial mode (tests, measurements);
         // REFORM_PRAQ_MEGA_PHANTOM=k makes every barrier wait for k CTAs that
@@ -2140,7 +2139,7 @@ struct Solver final : SolverBase {
             RB_CUDA_TRY(cudaGetDevice(&dev));
             RB_CUDA_TRY(cudaFuncGetAttributes(&fa, cluster_solve_kernel<Real>));
             RB_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-            *v = optin > int(fa.sharedSizeBytes) ? optin - int(fa.sharedSizeBytes) : 0;
+            *v = std::max(0, optin - int((fa.sharedSizeBytes + 15) / 16 * 16));   // (dynamic memory starts on 16 bytes)
             RB_CUDA_TRY(cudaFuncSetAttribute(cluster_solve_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, *v));
             return cudaFuncSetAttribute(cluster_solve_kernel<Real>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         }));
@@ -2173,16 +2172,29 @@ struct Solver final : SolverBase {
         cfg.numAttrs = 1;
     }
 
-    // A step of the cluster form costs its remote stores (r to 15 CTAs, a
-    // slot-1 value an edge); the graph's costs its launches.  Per solve, graph
-    // against cluster, FP32 / FP64: n = 700, m = 3,500 - / 0.65 against 0.36 ms;
-    // 1,000, 6,000 0.66 against 0.48 / 0.84 against 0.50; 2,000, 10,000 0.53
-    // against 0.46 / 0.68 against 0.45; 3,000, 12,000 0.64 against 0.63 / 0.80
-    // against 0.68; 3,000, 24,000 0.58 against 0.64 / 0.74 against 0.70; 5,000,
-    // 30,000 0.69 against 0.97 / 0.88 against 1.10.  (8 CTAs were slower than
-    // 16 from n = 1,500 up.)
-    static constexpr int kClusterNodes = sizeof(Real) == 4 ? 2048 : 3072;
-    static constexpr int kClusterEdges = sizeof(Real) == 4 ? 12288 : 24576;
+    // The forms' lines, from one table of all three at n = 300 to 5,000 and 0.5
+    // to 12 edges a node, uniform random, per solve.  A step of the single-CTA
+    // form costs its nodes four times its edges (a pass of 256 nodes is a chain
+    // of loads, one of 512 edges is not), one of the cluster form much the same
+    // with a sixteenth of the factor, its barriers and remote stores added; one of
+    // the graph costs two launches at these sizes.  So the lines lie at values of
+    // 4 n + m.  Single CTA against cluster, FP32: n = 700, m = 4,200 (7,000) 0.351
+    // against 0.353 ms, 1,250, 1,875 (6,875) 0.307 / 0.318, 1,000, 4,000 (8,000)
+    // 0.437 / 0.423, 1,750, 4,375 0.87 / 0.63; FP64: 500, 3,000 (5,000) 0.559 /
+    // 0.613, 600, 2,400 (4,800) 0.669 / 0.645, 700, 2,800 (5,600) 0.708 / 0.669,
+    // 1,000, 2,500 (6,500) 0.71 / 0.64.  Cluster against graph, FP32: 3,500,
+    // 14,000 (28,000) 0.529 / 0.543, 4,000, 10,000 (26,000) 0.426 / 0.443, 3,000,
+    // 18,000 (30,000) 0.585 / 0.557, 5,000, 12,500 (32,500) 0.781 / 0.734; FP64:
+    // 3,000, 24,000 (36,000) 0.966 / 1.067, 3,500, 21,000 (35,000) 0.954 / 0.996,
+    // 4,000, 24,000 (40,000) 1.044 / 1.015, 5,000, 7,500 0.633 / 0.594 (n is
+    // bounded as well there).  Single CTA against graph, where there is no cluster
+    // (no edges; 320 steps, one-shot): FP32 n = 2,500 1.23 / 1.34, 3,000 1.48 /
+    // 1.38; FP64 1,500 1.07 / 1.39, 2,500 1.48 / 1.38.
+    static constexpr long long kTinyWork = sizeof(Real) == 4 ? 7000 : 5000;
+    static constexpr long long kTinyWorkAlone = sizeof(Real) == 4 ? 10000 : 8000;
+    static constexpr long long kClusterWork = sizeof(Real) == 4 ? 28000 : 37000;
+    static constexpr int kClusterNodes = 4096;
+    long long step_work() const { return 4LL * n + m; }
 
     // Cut the instance over a cluster, if its bytes can fit one: the cut is
     // made on the device (it needs the run pointers) and read back.
@@ -2190,7 +2202,7 @@ struct Solver final : SolverBase {
         cluster_ctas = 0;
         const char* env = std::getenv("REFORM_PRAQ_CLUSTER");   // 0: never (tests, measurements)
         if (m == 0 || (env && !std::strcmp(env, "0"))) return cudaSuccess;
-        if (n > kClusterNodes || m > kClusterEdges) return cudaSuccess;
+        if (n > kClusterNodes || step_work() > kClusterWork) return cudaSuccess;
         int ctas = 0, room = 0;
         RB_CUDA_TRY(cluster_limits(&ctas, &room));
         const int real = int(sizeof(Real));
@@ -2224,16 +2236,14 @@ struct Solver final : SolverBase {
                                   hplan.max_nodes, hplan.max_edges, hplan.max_seconds, start, kTinyBlocks, budget_ns);
     }
 
-    // mode -1: automatic (the single-CTA form wherever the instance fits one
-    // CTA's shared memory, else the graph: per solve 0.21 against 0.60 ms at
-    // n = 200, m = 1,000, 0.36 against 0.64 at n = 700, m = 2,800, 1.63 against
-    // 2.01 at n = 1,500, m = 4,500, FP32, and 0.375 against 0.395 at n = 2,500,
-    // m = 3,000, about the largest that fits; the grid form was slower than
-    // the graph from n = 400 up); 0: the graph; 1: the single-CTA form when it
-    // fits, else the grid form; 2: the grid form.
+    // mode -1: automatic (the single-CTA form, the cluster form, the graph, by the
+    // lines above); 0: the graph; 1: the single-CTA form when the instance fits
+    // one CTA's shared memory, else the grid form (slower than the graph from n =
+    // 400 up); 2: the grid form.
     cudaError_t set_mega(int mode) {
         mega_mode = mode < 0 ? -1 : (mode > 2 ? 2 : mode);
-        tiny = tiny_fits && (mega_mode == 1 || mega_mode == -1);
+        const long long alone = cluster_ctas > 0 ? kTinyWork : kTinyWorkAlone;
+        tiny = tiny_fits && (mega_mode == 1 || (mega_mode == -1 && step_work() <= alone));
         clustered = !tiny && mega_mode == -1 && cluster_ctas > 0;
         mega = !tiny && mega_mode >= 1 && mega_grid > 0;
         if (mega && !bar.ptr) {

@@ -683,7 +683,7 @@ def test_convergence_trace_ring_wraps(native):
 
 
 @pytest.mark.parametrize("use_float32", [0, 1])
-@pytest.mark.parametrize("form,n,m", [("single-cta", 700, 2800), ("cluster", 1500, 6000)])
+@pytest.mark.parametrize("form,n,m", [("single-cta", 500, 2400), ("cluster", 1500, 6000)])
 @pytest.mark.parametrize("op_steps", [2, 16, 300])
 def test_budget_of_a_whole_solve_launch(native, use_float32, form, n, m, op_steps):
     """The forms that run many check blocks in one launch look at a wall-clock
@@ -866,3 +866,35 @@ def test_cluster_is_not_behind_the_graph_at_its_bound(native, use_float32, n, m)
                 best[mode] = min(best[mode], time.perf_counter() - start)
             assert mode == 0 or dev.launches() == 2
     assert best[-1] <= 1.01 * best[0]
+
+
+@pytest.mark.parametrize("use_float32", [0, 1])
+@pytest.mark.parametrize("line", ["single-cta", "cluster", "few-edges", "edgeless"])
+def test_forms_at_their_lines(native, use_float32, line):
+    """The automatic choice on both sides of its lines (values of 4 n + m, or
+    of n): the form shows in the launches of a solve, and every form gives the
+    graph's result bit for bit."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import Library
+    tiny, cluster = (7000, 28000) if use_float32 else (5000, 37000)
+    if line == "single-cta":
+        sizes = [(500, tiny - 2000, 2), (500, tiny - 1999, 0)]
+    elif line == "cluster":
+        n = 3001
+        sizes = [(n, cluster - 4 * n, 0), (n, cluster - 4 * n + 1, None)]
+    elif line == "few-edges":
+        sizes = [(4095, 517, 0), (4096, 1, 0), (4097, 517, None)]
+    else:
+        alone = 2500 if use_float32 else 2000
+        sizes = [(tiny // 4, 0, 2), (alone, 0, 2), (alone + 1, 0, None)]
+    p = Library().parameters(tolerance=1e-12, max_iter=80, use_float32=use_float32)
+    for n, m, form in sizes:
+        inst = qubo_uniform_edges(n, n, m) if m else QuboInstance(
+            "e", "e", n, np.random.default_rng(n).integers(-100, 101, n) * 1.0, np.zeros(0, np.int64),
+            np.zeros(0, np.int64), np.zeros(0))
+        (on, auto, launches), (_, graph, _) = (_praq_runs_any(inst, p, mode, runs=2) for mode in (-1, 0))
+        assert on == (form or 0) and (launches == 2) == (form is not None)
+        for a, ya in auto:
+            b, yb = graph[0]
+            assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
+            assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
