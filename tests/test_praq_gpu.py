@@ -898,3 +898,23 @@ def test_forms_at_their_lines(native, use_float32, line):
             b, yb = graph[0]
             assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
             assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
+
+
+@pytest.mark.parametrize("use_float32", [0, 1])
+def test_infinite_tolerance_makes_no_cut(native, use_float32):
+    """A run that ends at the check before the loop (relaxation_bounds) takes
+    the start step's five launches, not a cluster's cut at set-up, with the
+    bounds that a solve's first check finds."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import DeviceSolver, Library
+    inst = qubo_uniform_edges(6, 2000, 10_000)
+    lib = Library()
+    with DeviceSolver(inst, lib.parameters(tolerance=float("inf"), use_float32=use_float32)) as dev:
+        assert dev.run() == 0
+        a = dev.result()
+        assert dev.launches() == 5 and a.iterations == 0
+    with DeviceSolver(inst, lib.parameters(tolerance=1e-15, max_iter=16, use_float32=use_float32)) as dev:
+        dev.set_trace(4)
+        dev.run()
+        first = dev.trace()[0]
+    assert (first["lower"], first["upper"]) == (a.lower, a.upper)
