@@ -1122,10 +1122,10 @@ lower_kernel(Dev<Real> d, const Real* __restrict__ y, const Real* __restrict__ z
 
 // Both bounds of a check in one launch: they are independent, and short next to
 // a launch (N = 30, T = 75: 12.3 us against 10.7 + 8.7 as two; 60, 200: 25.0
-// against 14.8 + 12.8).  Taken up to kBoundsCtas CTAs, about five an SM: beyond,
-// the upper bound's long CTAs share the SMs with the other's (60, 365: 62.6
-// against 27.1 + 20.9 us; 100, 500: 124 against 51 + 41).
-constexpr int kBoundsCtas = 740;
+// against 14.8 + 12.8).  Taken up to kBoundsCtasPerSm CTAs an SM: beyond, the
+// upper bound's long CTAs share the SMs with the other's (60, 365: 62.6 against
+// 27.1 + 20.9 us; 100, 500: 124 against 51 + 41).
+constexpr int kBoundsCtasPerSm = 5;
 template <class Real>
 __global__ void __launch_bounds__(kAuxThreads)
 bounds_kernel(Dev<Real> d, const Real* __restrict__ x, const Real* __restrict__ y, const Real* __restrict__ z) {
@@ -1837,8 +1837,9 @@ struct Solver final : SolverBase {
             return c > n ? n : c;
         };
         int zrow = tp + 1, csize = cluster_for(tp + 1);
+        int sms = 0;
         {
-            int dev = 0, sms = 0;
+            int dev = 0;
             RB_CUDA_TRY(cudaGetDevice(&dev));
             RB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             d.zpair = sizeof(Real) == 8 && cluster_for(tp) > 1 && (long long)(tp / 2) * csize >= 2LL * sms ? 1 : 0;
@@ -1892,10 +1893,9 @@ struct Solver final : SolverBase {
         prm.omega0 = p.omega;
         prm.vanilla_solve = p.use_halpern ? 0 : 1;
         RB_CUDA_TRY(set_attributes());
-        choose_fused();
+        choose_fused(sms);
         // x, y, z (or x, y and z) per step; bounds, check; a restart step, check
         step_nodes = fused ? 2 : 3;
-        bound_nodes = tp + nblo <= kBoundsCtas ? 1 : 2;
         block_nodes = step_nodes * p.op_steps + bound_nodes + 1 + step_nodes + 1;
         RB_CUDA_TRY(init_mega());
         return cudaGetLastError();
@@ -2045,10 +2045,13 @@ struct Solver final : SolverBase {
     size_t fused_smem() const {
         return std::max(yz_smem, size_t(z_threads<Real>() / 32) * tp * sizeof(Real));
     }
-    void choose_fused() {
-        const char* env = std::getenv("REFORM_PRIA_FUSE");   // 0: never (tests, measurements)
-        fused = d.csize == 1 && !d.zpair && d.zstaged && fused_smem() <= size_t(z_slice_bytes<Real>()) &&
-                !(env && !std::strcmp(env, "0"));
+    void choose_fused(int sms) {
+        // REFORM_PRIA_FUSE=0: y and z, and the two bounds, a launch each, no chain
+        // (tests, measurements)
+        const char* env = std::getenv("REFORM_PRIA_FUSE");
+        const bool allowed = !(env && !std::strcmp(env, "0"));
+        fused = allowed && d.csize == 1 && !d.zpair && d.zstaged && fused_smem() <= size_t(z_slice_bytes<Real>());
+        bound_nodes = allowed && tp + nblo <= kBoundsCtasPerSm * sms ? 1 : 2;
         chained = fused && nd <= kChainEntries;
     }
 

@@ -585,3 +585,25 @@ def test_convergence_trace(native, mode):
     assert np.all(np.diff(tr["iteration"]) >= 0) and (tr["gap"][:-1] > 1e-7).all()
     for other in traces[1:]:
         assert other.tobytes() == tr.tobytes()
+
+
+@pytest.mark.parametrize("n,t,together", [(3, 17, True), (10, 25, True), (30, 75, True), (60, 365, False)])
+def test_fuse_off_separates_the_bounds_too(native, monkeypatch, n, t, together):
+    """REFORM_PRIA_FUSE=0 gives y, z and both bounds a launch each: a run that
+    ends at the check before the loop is x, y, z, upper, lower, check and the
+    result's own upper bound (7 launches), against x, yz, bounds, check and that
+    (5); the bounds agree bit for bit.
+    Instances whose bounds fill the device keep two launches."""
+    from reformulation_b200 import pria
+    inst = jrp_demand(20 + n, n, t)
+    out = []
+    for fuse in ("1", "0"):
+        monkeypatch.setenv("REFORM_PRIA_FUSE", fuse)
+        with pria.DeviceSolver(inst, pria.Library().parameters(64, 1e9), "fp64") as dev:
+            assert dev.run() == 0
+            r = dev.result()
+            assert r.iterations == 0
+            out.append((r.primal_objective, r.dual_objective, dev.launches()))
+    (pa, da, la), (pb, db, lb) = out
+    assert (pa, da) == (pb, db)
+    assert lb == 7 and (la == 5 if together else la > 5)
