@@ -918,3 +918,65 @@ def test_infinite_tolerance_makes_no_cut(native, use_float32):
         dev.run()
         first = dev.trace()[0]
     assert (first["lower"], first["upper"]) == (a.lower, a.upper)
+
+
+@pytest.mark.parametrize("use_float32", [0, 1])
+@pytest.mark.parametrize("n,m", [(400, 1600), (1500, 6000)], ids=["single-cta", "cluster"])
+def test_whole_solve_launches_resume_and_trace(native, use_float32, n, m):
+    """A solve of more check blocks than one launch takes (128) resumes from
+    global memory: three launches after the start point's, the graph's result
+    and convergence trace bit for bit."""
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import DeviceSolver, Library
+    inst = qubo_uniform_edges(5, n, m)
+    p = Library().parameters(tolerance=1e-16, max_iter=600, use_float32=use_float32, op_steps=2)
+    out = []
+    for mode in (-1, 0):
+        with DeviceSolver(inst, p) as dev:
+            dev.set_megakernel(mode)
+            dev.set_trace(1024)
+            for _ in range(2):
+                assert dev.run() == 1                  # the iteration limit
+                out.append((dev.result(want_x=True, want_dual=True), dev.trace()))
+                assert mode == 0 or dev.launches() == 4
+    (b, yb), tb = out[2]
+    assert b.iterations == 600 and len(tb) == 301
+    for (a, ya), ta in out:
+        assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
+        assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
+        assert ta.tobytes() == tb.tobytes()
+
+
+def test_cluster_solvers_on_threads(native):
+    """Eight solvers in the cluster form at once, each on a thread and a stream
+    of its own, beside a large one on the graph: each gives what it gives alone."""
+    import threading
+    from reformulation_b200.instances import qubo_uniform_edges
+    from reformulation_b200.praq import DeviceSolver, Library
+    lib = Library()
+    jobs = [(qubo_uniform_edges(k, 1200 + 150 * k, 5000 + 500 * k), lib.parameters(tolerance=1e-5, max_iter=4000))
+            for k in range(8)]
+    jobs.append((qubo_uniform_edges(9, 100_000, 800_000), lib.parameters(tolerance=1e-4)))
+    alone, together, solvers = [], [None] * len(jobs), [DeviceSolver(*job) for job in jobs]
+    for dev in solvers:
+        assert dev.run() in (0, 1)
+        alone.append(dev.result(want_dual=True))
+
+    def solve(k):
+        runs = []
+        for _ in range(4):
+            assert solvers[k].run() in (0, 1)
+            runs.append(solvers[k].result(want_dual=True))
+        together[k] = runs
+
+    threads = [threading.Thread(target=solve, args=(k,)) for k in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for (a, ya), runs in zip(alone, together):
+        for b, yb in runs:
+            assert (a.iterations, a.lower, a.upper) == (b.iterations, b.lower, b.upper)
+            assert np.array_equal(a.x, b.x) and np.array_equal(ya, yb)
+    for dev in solvers:
+        dev.close()
