@@ -425,8 +425,11 @@ __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, c
     }
 }
 
+// (The FP64 pull step reads two runs' bounds ahead of its wait; left to itself the
+// compiler holds it to five CTAs an SM and spills 48 bytes a thread.  Four, without:
+// n = 2e6, m = 2e7 76.2 to 74.6 ms a solve, 8e5, 8e6 26.2 to 26.0.)
 template <class Real, bool Reflect, bool Check, bool Wide = false, bool Pull = false>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, sizeof(Real) == 8 && Reflect && !Check && !Wide && Pull ? 4 : 0)
 node_kernel(Dev<Real> d, const Real* __restrict__ ys, const Real* __restrict__ yc, int step,
             int bounds_at_1, int gate) {
     node_kernel_tile<Real, Reflect, Check, Wide, Pull>(d, blockIdx.x, ys, yc, step, bounds_at_1, gate, PdlWait());
