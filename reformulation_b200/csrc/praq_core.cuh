@@ -137,7 +137,10 @@ struct alignas(16) Dev {   // (16-byte aligned: the batched engine copies descri
     Control* ctl;
 };
 
-constexpr int kWaitFirst = 1;   // a plain node step's gate: it reads what the kernel ahead writes
+// A step's gate: 0 a plain step; kWaitFirst a restart step (skipped unless one is
+// pending) that waits and decides before it reads, or a plain node step that
+// reads what the kernel ahead writes; kReadFirst a restart step that does not.
+constexpr int kWaitFirst = 1, kReadFirst = 2;
 __device__ __forceinline__ bool skip(const Control* c, int gate) {
     return c->terminated || (gate && !c->restart);
 }
@@ -360,10 +363,9 @@ template <class Real, bool Reflect, bool Check, bool Wide = false, bool Pull = f
 __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, const Real* ys, const Real* yc, int step,
                                                  int bounds_at_1, int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    // Ahead of the wait only in a chain, and only where the step is sure to be
-    // taken: a gated (restart) step leaves in most blocks, a finished instance
-    // of a batch in all.  A plain step with a gate (kWaitFirst) waits first too.
-    const bool early = Wait::kReadsEarly && !gate;
+    // Ahead of the wait only in a chain; not where much would be read for nothing
+    // (a restart step leaves in most blocks, a finished instance of a batch in all).
+    const bool early = Wait::kReadsEarly && gate != kWaitFirst;
     const int restart_gate = Reflect ? 0 : gate;
     if (!early) {
         wait();
@@ -443,7 +445,7 @@ template <class Real, bool Reflect, bool Check, bool Pull = false, int EPT = kEd
 __device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, const Real* ysrc, int step, int bounds_at_1,
                                                  int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    const bool early = Wait::kReadsEarly && (Reflect || !gate);   // (as in the node half)
+    const bool early = Wait::kReadsEarly && gate != kWaitFirst;   // (as in the node half)
     // the control block, the edges' constants, their dual and anchor: nothing
     // the kernel ahead (the node half) writes
     const bool off = skip(c, gate);
@@ -753,10 +755,10 @@ __device__ __forceinline__ bool mega_block_body(const Dev<Real>& d, const Params
         check_body(d.ctl, prm, d.scale, d.pnode, a.nb_node, d.pedge, a.nb_edge, d.plower, a.nb_node, 1);
     if (!sync()) return false;
     if (!d.ctl->restart) return true;   // uniform: the check above is the last writer
-    mega_node<Real, false, true, Wide>(d, a, d.u2s, d.u2s1, 0, 1);
+    mega_node<Real, false, true, Wide>(d, a, d.u2s, d.u2s1, 0, kReadFirst);
     if (!sync()) return false;
     if (d.m) {
-        mega_edge<Real, false, true>(d, a, d.u2s, 0, 1);
+        mega_edge<Real, false, true>(d, a, d.u2s, 0, kReadFirst);
         if (!sync()) return false;
     }
     if (blockIdx.x == 0)
@@ -1981,6 +1983,10 @@ struct Solver final : SolverBase {
     // edge bytes of a check block from which a first run waits for each check
     static constexpr double kLongBlockBytes = 400e6;
     static constexpr int kWaitedChecks = 10;
+    // edge bytes from which a restart step decides before it reads: what it reads
+    // for nothing shows from 28 MB (8.6 against 6.6 us a launch; at 8.4 MB 6.6 and
+    // 6.6), what it reads ahead saves a step that is taken 2 us
+    static constexpr double kLargeRestartBytes = 16e6;
     // The cluster form (cluster_solve_kernel): CTAs of its cluster (0: the
     // instance does not take it), its cut and dynamic shared memory.
     bool clustered = false;
@@ -2468,6 +2474,7 @@ struct Solver final : SolverBase {
         // where they are captured (1.19 against 1.24 ms).
         const bool chain = m > 0 || !capturing;
         const int first = m == 0 && chain ? kWaitFirst : 0;
+        const int gate = edge_bytes(m) > kLargeRestartBytes ? kWaitFirst : kReadFirst;
         for (int s = 0; s < op; ++s) {
             if (s + 1 < op) {
                 RB_TIMED(0, RB_CUDA_TRY(launch_ex(node_kernel<Real, true, false, W, P>, nb_node, kBlock, 0, chain, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, first)));
@@ -2480,8 +2487,8 @@ struct Solver final : SolverBase {
         RB_TIMED(4, RB_CUDA_TRY(launch_pdl(lower_kernel<Real, W, P>, nb_node, kBlock, stream, d, (const Real*)d.u2s, (const Real*)d.u2s1)));
         RB_TIMED(5, RB_CUDA_TRY(launch_pdl(check_kernel, 1, kCheckBlock, stream, d.ctl, prm, (const double*)d.scale, (const double*)d.pnode, nb_node,
                                                                 d.pedge, nb_edge, d.plower, nb_node, 1)));
-        RB_TIMED(6, RB_CUDA_TRY(launch_pdl(node_kernel<Real, false, true, W, P>, nb_node, kBlock, stream, d, (const Real*)d.u2s, (const Real*)d.u2s1, 0, 0, 1)));
-        if (m) RB_TIMED(7, RB_CUDA_TRY(launch_pdl(edge_kernel<Real, false, true, P>, nb_edge, kBlock, stream, d, (const Real*)d.u2s, 0, 0, 1)));
+        RB_TIMED(6, RB_CUDA_TRY(launch_pdl(node_kernel<Real, false, true, W, P>, nb_node, kBlock, stream, d, (const Real*)d.u2s, (const Real*)d.u2s1, 0, 0, gate)));
+        if (m) RB_TIMED(7, RB_CUDA_TRY(launch_pdl(edge_kernel<Real, false, true, P>, nb_edge, kBlock, stream, d, (const Real*)d.u2s, 0, 0, gate)));
         RB_TIMED(8, RB_CUDA_TRY(launch_pdl(check_kernel, 1, kCheckBlock, stream, d.ctl, prm, (const double*)d.scale, (const double*)d.pnode, nb_node,
                                                                 d.pedge, nb_edge, d.plower, nb_node, 2)));
         RB_CUDA_TRY(cudaMemcpyAsync(mirror, d.ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream));
