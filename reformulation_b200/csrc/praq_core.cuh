@@ -137,9 +137,8 @@ struct alignas(16) Dev {   // (16-byte aligned: the batched engine copies descri
     Control* ctl;
 };
 
-// A step's gate: 0 a plain step; kWaitFirst a restart step (skipped unless one is
-// pending) that waits and decides before it reads, or a plain node step that
-// reads what the kernel ahead writes; kReadFirst a restart step that does not.
+// A step's gate: 0 a plain step; else a restart step, skipped unless one is
+// pending: kWaitFirst waits and decides before it reads, kReadFirst does not.
 constexpr int kWaitFirst = 1, kReadFirst = 2;
 __device__ __forceinline__ bool skip(const Control* c, int gate) {
     return c->terminated || (gate && !c->restart);
@@ -365,11 +364,10 @@ __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, c
     const Control* c = d.ctl;
     // Ahead of the wait only in a chain; not where much would be read for nothing
     // (a restart step leaves in most blocks, a finished instance of a batch in all).
-    const bool early = Wait::kReadsEarly && gate != kWaitFirst;
-    const int restart_gate = Reflect ? 0 : gate;
+    const bool early = Wait::kReadsEarly && (Reflect || gate != kWaitFirst);   // (a plain step: known at compile time)
     if (!early) {
         wait();
-        if (skip(c, restart_gate)) return;
+        if (skip(c, gate)) return;
     }
     __shared__ double scratch[kNodeSums * 32];
     Real* stage = warp_stage<Real, stage_runs<Wide>()>();
@@ -392,7 +390,7 @@ __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, c
     }
     if (early) {
         wait();
-        if (skip(c, restart_gate)) return;
+        if (skip(c, gate)) return;
     }
     const Real s = scatter_at<Real, Real, Wide, Pull>(d, first, second, ys, yc, lane, stage);
     double acc[kNodeSums] = {0.0, 0.0, 0.0};
@@ -430,11 +428,11 @@ __device__ __forceinline__ void node_kernel_tile(const Dev<Real>& d, int tile, c
 // (The FP64 pull step reads two runs' bounds ahead of its wait; left to itself the
 // compiler holds it to five CTAs an SM and spills 48 bytes a thread.  Four, without:
 // n = 2e6, m = 2e7 76.2 to 74.6 ms a solve, 8e5, 8e6 26.2 to 26.0.)
-template <class Real, bool Reflect, bool Check, bool Wide = false, bool Pull = false>
+template <class Real, bool Reflect, bool Check, bool Wide = false, bool Pull = false, class Wait = PdlWait>
 __global__ void __launch_bounds__(kBlock, sizeof(Real) == 8 && Reflect && !Check && !Wide && Pull ? 4 : 0)
 node_kernel(Dev<Real> d, const Real* __restrict__ ys, const Real* __restrict__ yc, int step,
             int bounds_at_1, int gate) {
-    node_kernel_tile<Real, Reflect, Check, Wide, Pull>(d, blockIdx.x, ys, yc, step, bounds_at_1, gate, PdlWait());
+    node_kernel_tile<Real, Reflect, Check, Wide, Pull>(d, blockIdx.x, ys, yc, step, bounds_at_1, gate, Wait());
 }
 
 // Dual half of one PDHG step (solver.py:269-273, projection.py:16-42) in the
@@ -445,7 +443,7 @@ template <class Real, bool Reflect, bool Check, bool Pull = false, int EPT = kEd
 __device__ __forceinline__ void edge_kernel_tile(const Dev<Real>& d, int tile, const Real* ysrc, int step, int bounds_at_1,
                                                  int gate, Wait wait = Wait()) {
     const Control* c = d.ctl;
-    const bool early = Wait::kReadsEarly && gate != kWaitFirst;   // (as in the node half)
+    const bool early = Wait::kReadsEarly && (Reflect || gate != kWaitFirst);   // (as in the node half)
     // the control block, the edges' constants, their dual and anchor: nothing
     // the kernel ahead (the node half) writes
     const bool off = skip(c, gate);
@@ -793,7 +791,7 @@ mega_block_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant__ P
 // ---- the whole solve in one CTA's shared memory (a few thousand edges) ----
 // For a few hundred nodes the per-kernel graph and the grid form both wait on
 // latency: the generic tiles stage every gather through L2 in 256-thread
-// CTAs.  tiny_solve_kernel copies the instance into one 1024-thread CTA's
+// CTAs.  tiny_solve_kernel copies the instance into one kTinyThreads CTA's
 // shared memory and runs the start step, the check before the loop and up to
 // `max_blocks` check blocks there, with block barriers between phases, then
 // copies the iterates and the control block back.  It keeps the graph's
@@ -805,8 +803,7 @@ mega_block_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant__ P
 //   edges a kBlock apart, in order;
 // * per-tile check sums are block_sums over the half (butterfly in each
 //   warp, then the half's first warp adds its 8 warp totals in order), and
-//   check_body's row reductions see at most 256 rows, which 512 threads add
-//   in the order 256 threads do.
+//   check_body adds rows in the order of kCheckBlock threads, whatever the block.
 constexpr int kTinyThreads = 512;   // 128 registers a thread (1024 threads spill)
 constexpr int kTinyParts = kTinyThreads / kBlock;
 
@@ -2458,6 +2455,13 @@ struct Solver final : SolverBase {
             RB_TIMED(9, RB_CUDA_TRY(launch_mega()));
             return cudaMemcpyAsync(mirror, d.ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream);
         }
+        // With no edges a node step follows a node step, whose x it reads: a chain
+        // that waits before it reads where the steps are launched one by one (n =
+        // 5,000, 320 steps: 1.43 against 1.92 ms a one-shot solve), plain launches
+        // where they are captured (1.19 against 1.24 ms).
+        if (m == 0 && !capturing)
+            return wide ? enqueue_steps<true, false, PdlWait, PdlWaitFirst>()
+                        : enqueue_steps<false, false, PdlWait, PdlWaitFirst>();
         if (pull) return wide ? enqueue_steps<true, true>() : enqueue_steps<false, true>();
         if constexpr (sizeof(Real) == 8) {
             if (edges_wait) return wide ? enqueue_steps<true, false, PdlWaitFirst>() : enqueue_steps<false, false, PdlWaitFirst>();
@@ -2465,22 +2469,17 @@ struct Solver final : SolverBase {
         return wide ? enqueue_steps<true, false>() : enqueue_steps<false, false>();
     }
 
-    template <bool W, bool P, class EdgeWait = PdlWait>
+    template <bool W, bool P, class EdgeWait = PdlWait, class NodeWait = PdlWait>
     cudaError_t enqueue_steps() {
         const int op = int(p.op_steps);
-        // With no edges a node step follows a node step, whose x it reads: a chain
-        // that waits before it reads where the steps are launched one by one (n =
-        // 5,000, 320 steps: 1.43 against 1.92 ms a one-shot solve), plain launches
-        // where they are captured (1.19 against 1.24 ms).
         const bool chain = m > 0 || !capturing;
-        const int first = m == 0 && chain ? kWaitFirst : 0;
         const int gate = edge_bytes(m) > kLargeRestartBytes ? kWaitFirst : kReadFirst;
         for (int s = 0; s < op; ++s) {
             if (s + 1 < op) {
-                RB_TIMED(0, RB_CUDA_TRY(launch_ex(node_kernel<Real, true, false, W, P>, nb_node, kBlock, 0, chain, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, first)));
+                RB_TIMED(0, RB_CUDA_TRY(launch_ex(node_kernel<Real, true, false, W, P, NodeWait>, nb_node, kBlock, 0, chain, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, 0)));
                 if (m) RB_TIMED(1, RB_CUDA_TRY(launch_pdl(edge_plain_kernel<Real, P, EdgeWait>, P ? nb_edge_pull : nb_edge_push, kBlock, stream, d, (const Real*)nullptr, s, 0, 0)));
             } else {
-                RB_TIMED(2, RB_CUDA_TRY(launch_ex(node_kernel<Real, true, true, W, P>, nb_node, kBlock, 0, chain, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, first)));
+                RB_TIMED(2, RB_CUDA_TRY(launch_ex(node_kernel<Real, true, true, W, P, NodeWait>, nb_node, kBlock, 0, chain, stream, d, (const Real*)d.pred, (const Real*)d.pred1, s, 0, 0)));
                 if (m) RB_TIMED(3, RB_CUDA_TRY(launch_pdl(edge_kernel<Real, true, true, P, EdgeWait>, nb_edge, kBlock, stream, d, (const Real*)nullptr, s, 0, 0)));
             }
         }
@@ -2597,7 +2596,7 @@ struct Solver final : SolverBase {
     // L2 size.  REFORM_PRAQ_SLOT1=push|pull in the environment overrides the
     // choice (for tests and measurements).
     bool choose_pull(int64_t m_) const {
-        if (!allow_pull) return false;
+        if (!allow_pull || m_ == 0) return false;
         const char* env = std::getenv("REFORM_PRAQ_SLOT1");
         if (env && !std::strcmp(env, "push")) return false;
         if (env && !std::strcmp(env, "pull")) return true;
