@@ -142,12 +142,13 @@ REFORM_API int reform_praq_run_profiled(reform_praq_solver* solver, double* ms, 
  * check block per cooperative launch with its phases (node step; edge step;
  * lower bound; check; restart step) separated by grid barriers.  No
  * counterpart in the reference's praq-cuda; its pria-cuda has a megakernel
- * (PRIA_MEGA).  `mode` -1: automatic (the default: the single-CTA form
- * wherever the instance fits, 1.1-3x faster per solve than the graph; then, up
- * to 2,048 nodes and 12,288 edges in FP32 (3,072 and 24,576 in FP64), a solve
- * in one thread-block cluster's shared memory, 1.1-1.7x faster, reported as 0;
- * else the graph), 0: the graph, 1: the single-CTA form when the instance fits,
- * else the grid form, 2: the grid form.  The forms need the slot-1 push layout (edge arrays within twice the L2 size).
+ * (PRIA_MEGA).  `mode` -1: automatic (the default: the single-CTA form up to
+ * 4 n + m = 7,000 in FP32 and 5,000 in FP64, 1.2-2.9x faster per solve than the
+ * graph; then, up to 28,000 and 37,000 and 4,096 nodes, a solve in one
+ * thread-block cluster's shared memory, 1.02-1.8x faster, reported as 0; else
+ * the graph), 0: the graph, 1: the single-CTA form when the instance fits one
+ * CTA's shared memory, else the grid form, 2: the grid form.  The forms need the
+ * slot-1 push layout (edge arrays within twice the L2 size).
  * REFORM_PRAQ_MEGA=0|1 in the environment sets the mode at creation.
  * *active (may be NULL) receives the form later runs take: 1 the grid form, 2
  * the single-CTA form, 0 neither.  Results equal the graph's bit for bit

@@ -149,8 +149,9 @@ REFORM_API int reform_pria_run_profiled(reform_pria_solver* solver, double* ms, 
  * 145-312, PRIA_MEGA): a check block runs as ONE cooperative launch whose
  * phases (x; y and z; bounds; check; restart step) are separated by grid
  * barriers, in place of the captured graph.  `mode` 0: off (how a solver
- * starts: the graph measured faster at every size), -1: by size (on for at
- * most 16,384 packed entries, the reference's idea of small), 1: on whenever
+ * starts, and what to set to have that back: the graph is the faster form at
+ * every size, 1.7-2.6x at N = 3 to 30), -1: by size (on for at most 16,384
+ * packed entries, as this mode has always chosen), 1: on whenever
  * the instance allows it (every z period block within one CTA's shared
  * memory).  The environment variable REFORM_PRIA_MEGA=0|1 sets the mode at
  * creation.  *active (may be NULL) receives 1 when later runs take the

@@ -1685,11 +1685,11 @@ struct Solver final : SolverBase {
     long long nlaunch = 0, block_nodes = 0, step_nodes = 3, bound_nodes = 2;
     bool gated = false;   // the captured block is the conditional (gated) graph
     int runs = 0;
-    // The persistent kernel (mega_block_kernel) in place of the graph: chosen
-    // at set-up (mode -1: at most kMegaAutoEntries packed entries), or forced
-    // by set_mega; mega_grid resident CTAs of mega_smem bytes each.
+    // The persistent kernel (mega_block_kernel) in place of the graph: off at
+    // set-up, chosen by set_mega (mode -1: at most kMegaAutoEntries packed
+    // entries); mega_grid resident CTAs of mega_smem bytes each.
     bool mega = false;
-    int mega_mode = -1;              // -1 auto, 0 off, 1 on where the instance allows it
+    int mega_mode = 0;               // 0 off, -1 by size, 1 on where the instance allows it
     int mega_grid = 0;
     size_t mega_smem = 0;
     unsigned mega_phantom = 0;       // CTAs the barriers also wait for, never launched (fault injection)

@@ -166,10 +166,11 @@ class DeviceSolver:
         return _native.read_trace(self._lib.reform_praq_trace, self._h, getattr(self, "_trace_ring", 0), capacity)
 
     def set_megakernel(self, mode: int = -1) -> int:
-        """-1: automatic, 0: the per-kernel graph, 1: the persistent kernel's
-        single-CTA form where the instance fits, else its grid form, 2: the
-        grid form.  Returns the form later runs take: 0 the graph, 1 the grid
-        form, 2 the single-CTA form."""
+        """-1: automatic (the default: by size, the single-CTA form, a solve in one
+        thread-block cluster, the graph), 0: the per-kernel graph, 1: the persistent
+        kernel's single-CTA form where the instance fits, else its grid form, 2: the
+        grid form.  Returns the form later runs take: 1 the grid form, 2 the
+        single-CTA form, 0 the cluster or the graph."""
         active = ctypes.c_int(0)
         st = self._lib.reform_praq_set_megakernel(self._h, int(mode), ctypes.byref(active))
         if st != 0:

@@ -142,9 +142,9 @@ class DeviceSolver:
         return _native.read_trace(self._lib.reform_pria_trace, self._h, getattr(self, "_trace_ring", 0), capacity)
 
     def set_megakernel(self, mode: int = -1) -> bool:
-        """0: the per-kernel graph (how a solver starts), -1: the persistent
-        kernel for small instances, 1: wherever the instance allows it.  Returns whether
-        later runs take the persistent kernel."""
+        """0: the per-kernel graph (how a solver starts, and the faster form at
+        every size), -1: the persistent kernel for small instances, 1: wherever the
+        instance allows it.  Returns whether later runs take the persistent kernel."""
         active = ctypes.c_int(0)
         st = self._lib.reform_pria_set_megakernel(self._h, int(mode), ctypes.byref(active))
         if st != 0:
