@@ -927,11 +927,13 @@ __device__ __forceinline__ Acc tiny_run(const int* ptr, const Real* v, int i, in
 // runs from L2), so a warp with a few long runs adds them together, one after
 // the other.  Per solve with one node joined to every other, before this and
 // shared_long_run, now, and the graph, FP32 / FP64: n = 700, m = 1,700 (single
-// CTA) 0.97 / 1.84, 0.65 / 0.91, 0.85 / 1.45 ms; n = 2,000, m = 10,000 (cluster)
-// 18.8 / 22.4, 5.7 / 6.8, 6.4 / 11.6 ms.
+// CTA) 0.97 / 1.84, 0.68 / 0.93, 0.85 / 1.45 ms; n = 2,000, m = 10,000 (cluster)
+// 18.8 / 22.4, 5.6 / 6.9, 6.4 / 11.6 ms.  A call: with eight
+// copies of it in the kernel a solve behind a flushed L2 fetched up to 10 us more
+// instructions (n = 200 FP32 0.237 against 0.231 ms).
 constexpr int kLongRun = 64, kLongLanes = 4;
 template <class Acc, class Real>
-__device__ __forceinline__ Acc tiny_runs(const int* ptr, const Real* v, int i, int n, int m, int* status) {
+__device__ __noinline__ Acc tiny_runs(const int* ptr, const Real* v, int i, int n, int m, int* status) {
     Acc s = Acc(0);
     int k = 0, e = 0;
     if (i < n) {
@@ -1448,6 +1450,7 @@ constexpr int kClusterMax = 16;
 struct ClusterPlan {
     int node[kClusterMax + 1], edge[kClusterMax + 1], second[kClusterMax + 1];
     int max_nodes, max_edges, max_seconds;
+    int long_runs;   // some node's run has more than kLongRun values
 };
 static_assert(sizeof(ClusterPlan) <= 256, "read back through a pinned mirror slot");
 
@@ -1524,6 +1527,8 @@ __global__ void cluster_plan_kernel(int n, int m, int parts, int real, const int
         plan->max_edges = b;
         plan->max_seconds = c;
     }
+    const bool longs = any_long_run(row_ptr, col_ptr, n);
+    if (q == 0) plan->long_runs = longs ? 1 : 0;
 }
 
 __device__ __forceinline__ void cluster_barrier() {
@@ -1605,8 +1610,7 @@ cluster_solve_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant_
         w[e] = d.w[e0 + e];
         dst[e] = cluster_address(pred1_at, q) + unsigned(pos - second_cut[q]) * unsigned(sizeof(Real));
     }
-    __syncthreads();
-    const bool long_runs = any_long_run(rp, cp, nodes);
+    const bool long_runs = plan->long_runs != 0;
     auto check = [&](int mode) {
         if (rank == 0) {
             tiny_check(d.ctl, prm, d.scale, d.pnode, nb_node, d.pedge, nb_edge, d.plower, mode);
@@ -1615,8 +1619,8 @@ cluster_solve_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant_
         cluster_barrier();
     };
     if (start) {   // the start step with the bounds at the start point, and the check before the loop
-        tiny_node<Real, false, true>(d, d.pred, d.pred1, 0, 1, 0, nb_node, true, scratch, qout);
-        tiny_lower<Real>(d, d.pred, d.pred1, nb_node, true, scratch, qout);
+        tiny_node<Real, false, true>(d, d.pred, d.pred1, 0, 1, 0, nb_node, long_runs, scratch, qout);
+        tiny_lower<Real>(d, d.pred, d.pred1, nb_node, long_runs, scratch, qout);
         cluster_barrier();
         tiny_edge<Real, false, true>(d, d.pred, 0, 1, 0, nb_edge, scratch, qout);
         cluster_barrier();
@@ -1702,15 +1706,15 @@ cluster_solve_kernel(const __grid_constant__ Dev<Real> d, const __grid_constant_
         for (int e = tid; e < edges; e += kTinyThreads) d.pred[e0 + e] = pred[e];
         for (int k = tid; k < seconds; k += kTinyThreads) d.pred1[k0 + k] = pred1[k];
         cluster_barrier();
-        tiny_node<Real, true, true>(d, d.pred, d.pred1, op - 1, 0, 0, nb_node, true, scratch, qout);
+        tiny_node<Real, true, true>(d, d.pred, d.pred1, op - 1, 0, 0, nb_node, long_runs, scratch, qout);
         cluster_barrier();
         tiny_edge<Real, true, true>(d, nullptr, op - 1, 0, 0, nb_edge, scratch, qout);
         cluster_barrier();
-        tiny_lower<Real>(d, d.u2s, d.u2s1, nb_node, true, scratch, qout);
+        tiny_lower<Real>(d, d.u2s, d.u2s1, nb_node, long_runs, scratch, qout);
         cluster_barrier();
         check(1);
         if (d.ctl->restart) {   // uniform over the cluster
-            tiny_node<Real, false, true>(d, d.u2s, d.u2s1, 0, 0, 1, nb_node, true, scratch, qout);
+            tiny_node<Real, false, true>(d, d.u2s, d.u2s1, 0, 0, 1, nb_node, long_runs, scratch, qout);
             cluster_barrier();
             tiny_edge<Real, false, true>(d, d.u2s, 0, 0, 1, nb_edge, scratch, qout);
             cluster_barrier();
@@ -2223,7 +2227,7 @@ struct Solver final : SolverBase {
                              std::max(ctas, 1);
         if (ctas < 2 || share + double(n) * real > double(room)) return cudaSuccess;   // no cut can fit
         RB_CUDA_TRY(plan.alloc(1, stream));
-        cluster_plan_kernel<<<1, 32, 0, stream>>>(n, m, ctas, real, row_ptr.ptr, col_ptr.ptr, plan.ptr);
+        cluster_plan_kernel<<<1, kTinyThreads, 0, stream>>>(n, m, ctas, real, row_ptr.ptr, col_ptr.ptr, plan.ptr);
         RB_CUDA_TRY(cudaMemcpyAsync(mirror, plan.ptr, sizeof(ClusterPlan), cudaMemcpyDeviceToHost, stream));
         RB_CUDA_TRY(cudaStreamSynchronize(stream));
         std::memcpy(&hplan, mirror, sizeof(ClusterPlan));
